@@ -60,6 +60,9 @@ cudaError_t launch_fwd_generic(const FwdParams& p, cudaStream_t stream, long lon
 long long generic_grid_blocks(int B, int H, int S);
 cudaError_t launch_fwd_tcgen05(const FwdParams& p, int sm_count, cudaStream_t stream,
                                long long* launches);
+// The single-key-tile kernel (fwd_short.cu), S <= 128 and D <= 64.
+cudaError_t launch_fwd_short(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches);
+bool short_fits(int S, int D, float sm_scale);
 // The double-buffered-S family (D = 64, 128, 256), selected by launch_fwd_tcgen05.
 cudaError_t launch_fwd_tcgen05_db(const FwdParams& p, int sm_count, cudaStream_t stream,
                                   long long* launches);

@@ -2,10 +2,9 @@
 // (mma.sync m16n8k16, fp32 accumulate): the counterpart of the reference's
 // single-tile kernels _attn_fwd_small and _attn_fwd_small_causal
 // (ascend_rsfa/flash_attention_forward.py:26-159), which are latency- and
-// HBM-bound.  The dispatcher sends it the smallest tiles - head dimension 16 at
-// S <= 128, sequences of at most 64 keys at D <= 64 - where it measures faster
-// than the tcgen05 kernels, and every shape with a non-positive sm_scale, which
-// those are not built for.  It accepts any S >= 1, any D in {16,32,64,128,256} and
+// HBM-bound.  The dispatcher sends it every shape with a non-positive sm_scale,
+// which the other kernels are not built for; short sequences with a positive one
+// run on fwd_short.cu.  It accepts any S >= 1, any D in {16,32,64,128,256} and
 // any strides with a contiguous innermost dimension (the "force_path" option runs
 // it on every shape: the parity tests compare the two families that way); rows and
 // keys past S are predicated, which the reference does not do.

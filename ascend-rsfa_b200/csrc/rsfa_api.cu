@@ -82,7 +82,8 @@ int ensure_device(int device, DeviceState** out) {
 
 bool valid_head_dim(int D) { return D == 16 || D == 32 || D == 64 || D == 128 || D == 256; }
 
-// Kernel family by shape.  The tcgen05 kernels take everything they are instantiated for (sm_scale > 0)
+// Kernel family by shape (a single key tile then runs on fwd_short.cu in either family's place, see
+// short_fits; the times below are the families' own).  The tcgen05 kernels take everything they are instantiated for (sm_scale > 0)
 // except the smallest tiles: head dimension 16, and sequences of at most 64 keys at D <= 64, stay on
 // the short-sequence kernel, the counterpart of the reference's single-tile kernels for N_CTX <= 128
 // (:564).  Measured per call, host clock around call + synchronise / 4096 heads back to back:
@@ -372,7 +373,10 @@ int rsfa_fwd(const void* q, const void* k, const void* v, void* o, float* lse, i
     tile_of_path(path, S, D, causal, block_m, block_n, &bm, &bn);
     p.tile_n = bn;
   }
-  if (path == RSFA_PATH_TCGEN05)
+  // One key tile: the kernel for that, in place of either family (see RSFA_PATH_* in rsfa.h).
+  if (g_force_path.load() < 0 && p.variant < 0 && rsfa::short_fits(S, D, sm_scale))
+    e = rsfa::launch_fwd_short(p, d->sm_count, static_cast<cudaStream_t>(stream), &launches);
+  else if (path == RSFA_PATH_TCGEN05)
     e = rsfa::launch_fwd_tcgen05(p, d->sm_count, static_cast<cudaStream_t>(stream), &launches);
   else
     e = rsfa::launch_fwd_generic(p, static_cast<cudaStream_t>(stream), &launches);

@@ -356,8 +356,9 @@ EncodeTiledFn get_encode_fn() {
   return f;
 }
 
-// [B,H,S,D] tensor, 16-bit elements, as a 4-D map (D, S, H, B) with boxes of 64 x `box_rows`.
-bool make_map(CUtensorMap* map, const void* base, const FwdParams& p, const int64_t* st, int box_rows) {
+// [B,H,S,D] tensor, 16-bit elements, as a 4-D map (D, S, H, B) with boxes of `box_cols` x `box_rows`.
+bool make_map_boxed(CUtensorMap* map, const void* base, const FwdParams& p, const int64_t* st, int box_cols, int box_rows,
+                    CUtensorMapSwizzle swizzle) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return false;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(p.D), static_cast<cuuint64_t>(p.S),
@@ -369,13 +370,16 @@ bool make_map(CUtensorMap* map, const void* base, const FwdParams& p, const int6
   };
   const cuuint64_t strides[3] = {stride_bytes(st[2], p.S, p.D), stride_bytes(st[1], p.H, static_cast<int64_t>(p.S) * p.D),
                                  stride_bytes(st[0], p.B, static_cast<int64_t>(p.H) * p.S * p.D)};
-  const cuuint32_t box[4] = {64u, static_cast<cuuint32_t>(box_rows), 1u, 1u};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows), 1u, 1u};
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   const CUresult r = enc(map, p.bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                          const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                         swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
+}
+// ... with the 64-column, 128-byte-swizzled boxes of the tcgen05 kernels.
+bool make_map(CUtensorMap* map, const void* base, const FwdParams& p, const int64_t* st, int box_rows) {
+  return make_map_boxed(map, base, p, st, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace

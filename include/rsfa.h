@@ -41,6 +41,12 @@ extern "C" {
 /* Kernel families a call can be routed to (see rsfa_select_path). */
 #define RSFA_PATH_GENERIC 0 /* mma.sync kernel: any S, D in {16,32,64,128,256}; the smallest tiles, scale <= 0 */
 #define RSFA_PATH_TCGEN05 1 /* warp-specialised tcgen05 / TMEM / TMA kernel                         */
+/*
+ * Sequences of one key tile - S <= 128 at D <= 64, S <= 64 at D = 128, sm_scale > 0 - run on a kernel of
+ * their own (TMA-fed, warp-level MMA, csrc/fwd_short.cu) whichever of the two families their size belongs
+ * to, unless "force_path" or "tcgen05_variant" asks for a particular kernel.  rsfa_select_path,
+ * rsfa_get_tiling and rsfa_work_items name the family and its tile and count of items by size alone.
+ */
 
 /*
  * Forward attention on device tensors.  Replaces _attention.forward (:547-616)

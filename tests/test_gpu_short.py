@@ -1,0 +1,83 @@
+"""The single-key-tile kernel (csrc/fwd_short.cu) on a B200: edges of its strips of 16 rows, its steps of 32
+keys and its ring plan, every head dimension it takes, against the fp32 oracle; storage orders against the
+general mma.sync kernel."""
+import math
+
+import pytest
+import torch
+
+from oracle.attention_ref import attention_fp32, make_inputs
+
+pytestmark = pytest.mark.gpu
+
+UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}   # unit roundoff
+
+
+@pytest.fixture(scope="module")
+def fa(cuda_device):
+    import ascend_rsfa.flash_attention_forward as mod
+
+    return mod
+
+
+def bound(v, dtype):
+    # every weight and every result is rounded once to 16 bits, the weights sum to one:
+    # |error| <= u * max|v| + u * |o|, plus fp32 sums of at most 128 terms
+    return 2 * UNIT[dtype] * float(v.float().abs().max()) + 1e-4
+
+
+@pytest.mark.parametrize("D", [16, 32, 64, 128])
+@pytest.mark.parametrize("heads", [(1, 1), (3, 5), (37, 33)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_lengths_at_the_edges_of_strips_and_steps(fa, cuda_device, D, heads, dtype):
+    B, H = heads
+    for S in (1, 15, 16, 17, 32, 33, 63, 64) + ((65, 97, 112, 113, 127, 128) if D <= 64 else ()):
+        q, k, v = make_inputs(B, H, S, D, seed=S + D, dtype=dtype)
+        for causal in (False, True):
+            n0 = fa.launch_count()
+            o, lse = fa.attention_with_lse(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), causal,
+                                           1.0 / math.sqrt(D))
+            torch.cuda.synchronize()
+            fa.device_status()
+            assert fa.launch_count() - n0 == 1
+            ref, lse_ref = attention_fp32(q, k, v, causal, 1.0 / math.sqrt(D), return_lse=True)
+            assert float((o.cpu().float() - ref).abs().max()) <= bound(v, dtype), (S, causal)
+            assert torch.allclose(lse.cpu(), lse_ref, atol=1e-4, rtol=1e-4), (S, causal)
+
+
+@pytest.mark.parametrize("S,D", [(64, 64), (50, 128), (100, 32), (128, 16), (23, 64)])
+def test_storage_orders_agree_with_the_general_kernel(fa, cuda_device, S, D):
+    B, H = 5, 6
+    g = torch.Generator(device=cuda_device).manual_seed(S)
+    rand = lambda *shape: torch.randn(shape, generator=g, device=cuda_device).half()  # noqa: E731
+    forms = {
+        "bshd": [rand(B, S, H, D).transpose(1, 2) for _ in range(3)],
+        "hbsd": [rand(H, B, S, D).transpose(0, 1) for _ in range(3)],
+        "packed qkv": list(rand(B, S, 3, H, D).permute(2, 0, 3, 1, 4).unbind(0)),
+        "padded rows": [rand(B, H, S, D + 8)[..., :D] for _ in range(3)],
+        "sliced heads": [rand(B, 2 * H, S + 3, D)[:, 1::2, 2:S + 2] for _ in range(3)],
+        "one batch, odd stride": [rand(3 * H * S * D + 24)[:H * S * D].view(1, H, S, D) for _ in range(3)],
+    }
+    for name, (q, k, v) in forms.items():
+        for causal in (False, True):
+            o = fa.attention(q, k, v, causal, 0.2, 64, 64)
+            fa.set_option("force_path", 0)
+            try:
+                general = fa.attention(q, k, v, causal, 0.2, 64, 64)
+            finally:
+                fa.set_option("force_path", -1)
+            torch.cuda.synchronize()
+            assert o.stride() == general.stride(), name
+            assert float((o.float() - general.float()).abs().max()) <= bound(v, torch.float16), (name, causal)
+
+
+def test_rows_with_infinite_scores_and_nan_stay_where_they_are(fa, cuda_device):
+    # a NaN or an infinity in one query row reaches that row only; in a key or a value, every row that sees it
+    q, k, v = make_inputs(2, 3, 40, 64, seed=3)
+    q[0, 0, 5, 0] = float("nan")
+    q[1, 2, 7, 3] = float("inf")
+    o = fa.attention(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), False, 0.125, 64, 64).cpu().float()
+    ref = attention_fp32(q, k, v, False, 0.125)
+    bad = torch.isnan(ref).any(-1)
+    assert torch.equal(torch.isnan(o).any(-1), bad) and bool(bad[0, 0, 5]) and int(bad.sum()) <= 2
+    assert float((o - ref)[~bad].abs().max()) <= bound(v, torch.float16)
