@@ -10,10 +10,10 @@ return types —
     get_num_compute_cores()                                             (:19)
 
 — on [B, H, S, D] fp16 (or bf16) CUDA tensors.  The work is done by hand-written
-sm_100a kernels in librsfa_b200.so, reached through its C ABI with ctypes; this
-file only validates, allocates the output like the reference does
-(``torch.empty_like(q)``, :558) and passes raw pointers, strides and the current
-CUDA stream.  There is no Triton, no PyTorch math and no CPU path here: without
+sm_100a kernels in librsfa_b200.so, reached through its C ABI - from a small
+native extension for the ordinary call, with ctypes for the rest; this file only
+validates, allocates the output like the reference does (``torch.empty_like(q)``,
+:558) and passes raw pointers, strides and the current CUDA stream.  There is no Triton, no PyTorch math and no CPU path here: without
 the library, or on a non-CUDA tensor, the call raises.
 
 Differences from the reference, all on purpose:
@@ -31,7 +31,14 @@ import torch
 
 from . import _capi
 
+try:
+    from . import _rsfa_torch
+except ImportError as e:
+    raise ImportError("the PyTorch side of the operator call is not built for this torch: run "
+                      "`python ascend-rsfa_b200/build.py` (%s)" % e) from e
+
 _lib = _capi.load()
+_rsfa_torch.bind(ctypes.cast(_lib.rsfa_fwd, ctypes.c_void_p).value)
 
 DEVICE = "cuda"
 _DTYPES = {torch.float16: _capi.RSFA_DTYPE_F16, torch.bfloat16: _capi.RSFA_DTYPE_BF16}
@@ -85,6 +92,13 @@ def _dense(t):
 
 
 def _forward(q, k, v, causal, sm_scale, BM, BN, want_lse):
+    # The ordinary call - dense CUDA tensors on the current device, plain argument types, no modes or
+    # transforms - in native code, 10 us of Python less (csrc/torch_binding.cpp); None: not ordinary.
+    done = _rsfa_torch.forward(q, k, v, causal, sm_scale, BM, BN, want_lse)
+    if type(done) is tuple:
+        return done
+    if done is not None:
+        _capi.check(done, "rsfa_fwd")
     assert q.shape[-1] == k.shape[-1] and k.shape[-1] == v.shape[-1]
     assert q.shape[-1] in {16, 32, 64, 128, 256}
     if q.dim() != 4 or q.shape != k.shape or q.shape != v.shape:

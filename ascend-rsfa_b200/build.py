@@ -2,6 +2,9 @@
 
     python ascend-rsfa_b200/build.py [--force] [--verbose] [--trace]
 
+Beside the library, the PyTorch side of the operator call (csrc/torch_binding.cpp) is
+compiled against the installed torch into ascend_rsfa/_rsfa_torch*.so.
+
 The library lands beside the Python module that loads it
 (ascend_rsfa/librsfa_b200.so) together with a stamp file holding a hash of the
 sources, headers and compiler flags it was built from; a rebuild happens when
@@ -15,10 +18,12 @@ into a buffer given through the "trace_ptr" option.  The per-role cycle tables
 under profiles/ come from that build; the product library has no trace code.
 """
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -30,6 +35,49 @@ FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-cudart", "static",
 ]
+
+
+BINDING = "torch_binding.cpp"
+OUT_BINDING = os.path.join(HERE, "ascend_rsfa", "_rsfa_torch" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def binding_command():
+    """The g++ command line of the PyTorch extension: headers and libraries of the torch in use."""
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
+    inc = [sysconfig.get_paths()["include"], os.path.join(torch_dir, "include"),
+           os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+    lib = os.path.join(torch_dir, "lib")
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1"] +
+            ["-I" + i for i in inc] + [os.path.join(CSRC, BINDING), "-o", OUT_BINDING, "-L" + lib] +
+            ["-l" + n for n in ("torch_python", "torch", "torch_cpu", "c10_cuda", "c10")])
+
+
+def binding_hash():
+    """Hash of the extension's source, its command line and the torch and Python it is built against."""
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    h = hashlib.sha256()
+    for f in (os.path.join(CSRC, BINDING), os.path.join(torch_dir, "version.py")):
+        with open(f, "rb") as fh:
+            h.update(fh.read() + b"\0")
+    h.update(" ".join(binding_command()).encode() + sys.version.encode())
+    return h.hexdigest()
+
+
+def build_binding(force=False):
+    stamp = OUT_BINDING + ".stamp"
+    want = binding_hash()
+    if not force and os.path.exists(OUT_BINDING) and os.path.exists(stamp):
+        with open(stamp) as fh:
+            if fh.read().strip() == want:
+                return OUT_BINDING
+    r = subprocess.run(binding_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError("g++ failed on " + BINDING)
+    with open(stamp, "w") as fh:
+        fh.write(want + "\n")
+    return OUT_BINDING
 
 
 def find_nvcc():
@@ -60,6 +108,7 @@ def stale(out, flags):
 def build(force=False, verbose=False, trace=False):
     out = OUT_TRACE if trace else OUT
     flags = FLAGS + (["-DRSFA_TRACE"] if trace else [])
+    build_binding(force)
     if not force and not stale(out, flags):
         return out
     nvcc = find_nvcc()
