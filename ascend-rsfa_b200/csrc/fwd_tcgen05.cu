@@ -11,8 +11,14 @@
 // diagonal (or the ragged end of the sequence) — with the state in registers and
 // the accumulator in tensor memory.
 //
-// One CTA owns kNT query tiles of 128 rows ("Q tiles") of one (batch, head) and
-// sweeps the keys in tiles of 128.  Roles:
+// One CTA owns kNT query tiles of 128 rows ("Q tiles") and sweeps the keys in
+// tiles of 128.  As a rule the Q tiles are neighbours in one (batch, head) and share
+// its K/V tiles (kPair).  At D = 128 there are two other forms, in which each Q tile
+// has K/V tiles of its own: two heads of one key tile each (kTwoHeads: with one head
+// per item half the CTA was idle and 4096 heads of S = 128 took 86-97 us, 3.4 us per
+// item; now 81, the time their bytes take), and the same 128 rows twice with the key
+// tiles dealt out in turn and the two partial results merged in the epilogue
+// (kSplitKeys, see split_keys_pays).  Roles:
 //   warps 0..3   softmax group 0: one thread per row of Q tile 0
 //   warps 4..7   softmax group 1: one thread per row of Q tile 1
 //   warp  8      TMA producer (one lane): Q tiles once per work item, K/V tiles
@@ -59,18 +65,27 @@ constexpr int kTmaWarp = 8;
 constexpr int kMmaWarp = 9;
 constexpr int kTmemCols = 512;
 
-template <int D>
+// What the two Q tiles of a work item are.
+enum : int {
+  kPair = 0,       // two neighbouring blocks of 128 rows of one head; they share its K/V tiles
+  kTwoHeads = 1,   // S <= 128: the single block of each of two heads, each with its own K/V tile
+  kSplitKeys = 2   // the same 128 rows twice: tile t takes key tiles t, t + 2, ...; O_0 and O_1 are merged
+};
+
+template <int D, int kMode>
 struct Cfg {
   static constexpr int kBoxes = D / 64;                       // 64-column TMA boxes per row
   static constexpr int kQTileBytes = kTileM * D * 2;
+  static constexpr int kQBufs = (kMode == kSplitKeys) ? 1 : kNT;   // its two tiles have the same rows
   static constexpr int kKvTileBytes = kTileN * D * 2;
   static constexpr int kStages = (D == 128) ? 4 : 6;
   static constexpr int kQBoxBytes = kTileM * 128;             // 128 rows x 128 B
   static constexpr int kKvBoxBytes = kTileN * 128;
   static constexpr int kStageBytes = kTileM * 128;            // epilogue staging: 128 rows x 64 columns
-  static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4;
-  static constexpr int kSmemBytes = kNT * kQTileBytes + kStages * kKvTileBytes + kNT * kStageBytes + 1024 /*align*/ +
-                                    kNumBarriers * 8 + 64;
+  static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4 + 2;
+  static constexpr int kMlBytes = (kMode == kSplitKeys) ? kNT * kTileM * 8 : 0;   // (m, l) of every row, twice
+  static constexpr int kSmemBytes = kQBufs * kQTileBytes + kStages * kKvTileBytes + kNT * kStageBytes + 1024 /*align*/ +
+                                    kNumBarriers * 8 + 64 + kMlBytes;
   __host__ __device__ static constexpr int kColS(int t) { return t * kTileN; }
   __host__ __device__ static constexpr int kColO(int t) { return 2 * kTileN + t * D; }
 };
@@ -82,15 +97,15 @@ __device__ __forceinline__ int num_kv_tiles(int row0, int S, int causal) {
   return (last_key + kTileN - 1) / kTileN;
 }
 
-template <int D, bool kBf16>
+template <int D, bool kBf16, int kMode>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, const SchedInfo sched) {
-  using C = Cfg<D>;
+  using C = Cfg<D, kMode>;
   extern __shared__ uint8_t smem_raw[];
   // 128-byte-swizzled tiles need 1024-byte alignment.
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = smem_base;
-  const uint32_t sKV = sQ + kNT * C::kQTileBytes;
+  const uint32_t sKV = sQ + C::kQBufs * C::kQTileBytes;
   const uint32_t sStage = sKV + C::kStages * C::kKvTileBytes;   // one staging buffer per softmax group
   const uint32_t sBar = sStage + kNT * C::kStageBytes;
   // barrier addresses
@@ -106,18 +121,26 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   auto bar_pv0_done = [&](int t) { return sBar + 8u * (7 * kNT + 2 * C::kStages + t); };
   const uint32_t bar_sched_full0 = sBar + 8u * (8 * kNT + 2 * C::kStages);  // 2 slots
   const uint32_t bar_sched_empty0 = bar_sched_full0 + 16u;                   // 2 slots
+  // kSplitKeys: (m, l) of both tiles are in shared memory / both groups have read O_0 and O_1
+  const uint32_t bar_ml_ready = bar_sched_empty0 + 16u;
+  const uint32_t bar_o_read = bar_ml_ready + 8u;
   const uint32_t misc = sBar + 8u * C::kNumBarriers;
-  // misc words: [0] TMEM base, [1] abort flag, [2..3] scheduler ring
+  // misc words: [0] TMEM base, [1] abort flag, [2..3] scheduler ring, then for kSplitKeys (m, l) per row
   uint8_t* misc_ptr = smem_raw + (misc - smem_u32(smem_raw));
   volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(misc_ptr);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc_ptr + 4);
   volatile int* sched_ring = reinterpret_cast<volatile int*>(misc_ptr + 8);
+  volatile float2* s_ml = reinterpret_cast<volatile float2*>(misc_ptr + 64);   // [kNT][kTileM]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint64_t wait_ns = p.wait_limit_ns;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
+    if constexpr (kMode == kSplitKeys) {
+      mbar_init(bar_ml_ready, kNT * kTileM);
+      mbar_init(bar_o_read, kNT * kTileM);
+    }
     for (int t = 0; t < kNT; ++t) {
       mbar_init(bar_q_full(t), 1);
       mbar_init(bar_q_empty(t), 1);
@@ -157,12 +180,25 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   griddep_wait();
 
   const int S = p.S;
-  // work item -> (head, first row).  Causal: heaviest (last) row block first.
-  auto decode = [&](int item, int& bh, int& row0) {
-    int blk;
-    sched_decode(sched, p.causal, item, bh, blk);
-    row0 = blk * (kNT * kTileM);
+  // work item -> (head, first row) of Q tile t.  Causal: heaviest (last) row block first.
+  auto decode = [&](int item, int t, int& bh, int& row0) {
+    if constexpr (kMode == kTwoHeads) {
+      bh = item * kNT + t;
+      row0 = 0;
+    } else {
+      int blk;
+      sched_decode(sched, p.causal, item, bh, blk);
+      row0 = kMode == kPair ? blk * (kNT * kTileM) + t * kTileM : blk * kTileM;
+    }
   };
+  // number of key tiles of Q tile t (0: it has nothing to do in this item)
+  auto tile_steps = [&](int t, int bh, int row0) -> int {
+    if (kMode == kTwoHeads && bh >= p.B * p.H) return 0;
+    const int n = num_kv_tiles(row0, S, p.causal);
+    return kMode == kSplitKeys ? (n + 1 - t) / 2 : n;
+  };
+  // key tile of step j of Q tile t
+  auto key_tile = [](int t, int j) -> int { return kMode == kSplitKeys ? 2 * j + t : j; };
 
   // setmaxnreg is warpgroup-aligned: every warp of a warpgroup must execute the SAME instruction,
   // so the third warpgroup lowers its budget before it splits into roles.
@@ -194,22 +230,34 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           griddep_launch_dependents();   // the queue is empty: the next kernel on the stream may set up
           break;
         }
-        int bh, row0;
-        decode(item, bh, row0);
-        const int b = bh / p.H, h = bh - b * p.H;
+        int tb[kNT], th[kNT], trow[kNT], n[kNT];   // batch, head, first row and steps of each Q tile
         int nmax = 0;
-        for (int t = 0; t < kNT; ++t) nmax = max(nmax, num_kv_tiles(row0 + t * kTileM, S, p.causal));
+#pragma unroll
+        for (int t = 0; t < kNT; ++t) {
+          if (kMode == kPair && t > 0) {   // the same head, the next block of rows
+            tb[t] = tb[0];
+            th[t] = th[0];
+            trow[t] = trow[0] + t * kTileM;
+            n[t] = num_kv_tiles(trow[t], S, p.causal);
+          } else {
+            int bh;
+            decode(item, t, bh, trow[t]);
+            tb[t] = bh / p.H;
+            th[t] = bh - tb[t] * p.H;
+            n[t] = tile_steps(t, bh, trow[t]);
+          }
+          nmax = max(nmax, n[t]);
+        }
 
         auto load_q = [&](int t) -> bool {
           if (!mbar_wait(bar_q_empty(t), (item_count & 1) ^ 1, abort_flag, wait_ns, kTagQEmpty)) return false;
           RSFA_TRACE_EV(0x100 + t);
           mbar_arrive_expect_tx(bar_q_full(t), C::kQTileBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
-            tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64,
-                        row0 + t * kTileM, h, b);
+            tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64, trow[t], th[t], tb[t]);
           return true;
         };
-        auto load_kv = [&](const CUtensorMap* map, int j) -> bool {
+        auto load_kv = [&](const CUtensorMap* map, int t, int j) -> bool {
           if (static_cast<int>(kv_count) == p.test_drop_load) {   // test hook: this tile is never announced
             ++kv_count;
             return true;
@@ -221,20 +269,36 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           mbar_arrive_expect_tx(bar_kv_full(s), C::kKvTileBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
             tma_load_4d(sKV + s * C::kKvTileBytes + bx * C::kKvBoxBytes, map, bar_kv_full(s), bx * 64,
-                        j * kTileN, h, b);
+                        key_tile(t, j) * kTileN, th[t], tb[t]);
           ++kv_count;
           return true;
         };
-        // K_0 first: its ring slot frees up while the previous item drains.  Then the Q tiles, which
-        // wait for that item's last QK^T, and only then V_0, whose slot frees up last of all: behind
-        // V_0 the Q loads, which come from DRAM, started 2000 clk later than they could.
-        if (nmax > 0) ok = load_kv(&maps.k, 0);
-        if (ok) ok = load_q(0);
-        if (ok) ok = load_q(1);
-        if (ok && nmax > 0) ok = load_kv(&maps.v, 0);
-        for (int j = 1; ok && j < nmax; ++j) {
-          ok = load_kv(&maps.k, j);
-          if (ok) ok = load_kv(&maps.v, j);
+        if constexpr (kMode == kPair) {
+          // K_0 first: its ring slot frees up while the previous item drains.  Then the Q tiles, which
+          // wait for that item's last QK^T, and only then V_0, whose slot frees up last of all: behind
+          // V_0 the Q loads, which come from DRAM, started 2000 clk later than they could.
+          if (nmax > 0) ok = load_kv(&maps.k, 0, 0);
+          if (ok) ok = load_q(0);
+          if (ok) ok = load_q(1);
+          if (ok && nmax > 0) ok = load_kv(&maps.v, 0, 0);
+          for (int j = 1; ok && j < nmax; ++j) {
+            ok = load_kv(&maps.k, 0, j);
+            if (ok) ok = load_kv(&maps.v, 0, j);
+          }
+        } else {
+          // Every Q tile has K/V tiles of its own, in the ring in the order in which the MMA warp uses them:
+          // K^0_0 K^1_0, then per step V^0_j K^0_{j+1} V^1_j K^1_{j+1}.  A Q tile without work still gets its
+          // Q (rows of a head past the last one read as zeros), so that its barriers keep step.
+          for (int t = 0; ok && t < kNT; ++t) {
+            if (n[t] > 0) ok = load_kv(&maps.k, t, 0);
+            if (ok && t < C::kQBufs) ok = load_q(t);
+          }
+          for (int j = 0; ok && j < nmax; ++j) {
+            for (int t = 0; ok && t < kNT; ++t) {
+              if (j < n[t]) ok = load_kv(&maps.v, t, j);
+              if (ok && j + 1 < n[t]) ok = load_kv(&maps.k, t, j + 1);
+            }
+          }
         }
         ++item_count;
       }
@@ -266,12 +330,18 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
         if (item >= sched.total_items) break;
         RSFA_TRACE_EV(0xa000);   // item known
-        int bh, row0;
-        decode(item, bh, row0);
         int n[kNT];
         int nmax = 0;
-        for (int t = 0; t < kNT; ++t) {
-          n[t] = num_kv_tiles(row0 + t * kTileM, S, p.causal);
+        int bh, row0;
+        decode(item, 0, bh, row0);
+        n[0] = tile_steps(0, bh, row0);
+        nmax = n[0];
+#pragma unroll
+        for (int t = 1; t < kNT; ++t) {
+          if (kMode == kPair)
+            n[t] = num_kv_tiles(row0 + t * kTileM, S, p.causal);
+          else
+            n[t] = tile_steps(t, kMode == kTwoHeads ? bh + t : bh, row0);
           nmax = max(nmax, n[t]);
         }
         // S_t = Q_t K^T : both operands K-major, 64-column boxes, 8-row atoms of 1024 B.  A step
@@ -281,7 +351,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         // instruction (batched: +3 % at D = 128, +4 % at D = 64).  A commit of 0 means none.
         auto issue_qk = [&](int t, uint32_t kslot, uint32_t commit_a, uint32_t commit_b, uint32_t commit_c = 0u,
                             uint32_t commit_d = 0u) {
-          const uint64_t qd = desc_q0 + static_cast<uint64_t>((t * C::kQTileBytes) >> 4);
+          const uint64_t qd = desc_q0 + static_cast<uint64_t>(((C::kQBufs == 1 ? 0 : t) * C::kQTileBytes) >> 4);
           const uint64_t kd = desc_k0 + static_cast<uint64_t>((kslot * C::kKvTileBytes) >> 4);
           if (elect_one()) {
 #pragma unroll
@@ -314,6 +384,63 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           return wait_all(bar_kv_full(idx % C::kStages), (idx / C::kStages) & 1, kTagKvFull);
         };
 
+        if constexpr (kMode != kPair) {
+          // K/V tiles of their own for each Q tile: a ring entry is read by one batch of MMAs and given back
+          // behind it.
+          auto next_kv = [&]() -> bool {
+            if (!wait_kv(kv_count)) return false;
+            tc_fence_after_sync();
+            return true;
+          };
+          // Q buffer to give back behind QK^T of step j of tile t (0: none): its own one behind its last step,
+          // the shared one behind the last QK^T of the item.
+          auto q_release = [&](int t, int j) -> uint32_t {
+            if (j + 1 != n[t]) return 0u;
+            if (C::kQBufs == kNT) return bar_q_empty(t);
+            return t == (n[1] == n[0] ? 1 : 0) ? bar_q_empty(0) : 0u;
+          };
+          for (int t = 0; ok && t < kNT; ++t) {
+            if (n[t] > 0) {
+              ok = next_kv();
+              if (ok && t < C::kQBufs) ok = wait_all(bar_q_full(t), item_count & 1, kTagQFull);
+              if (!ok) break;
+              tc_fence_after_sync();
+              issue_qk(t, kv_count % C::kStages, bar_s_full(t), q_release(t, 0), bar_kv_empty(kv_count % C::kStages));
+              ++kv_count;
+            } else if (t < C::kQBufs) {
+              ok = wait_all(bar_q_full(t), item_count & 1, kTagQFull);
+              if (!ok) break;
+              umma_commit_elect(bar_q_empty(t));
+            }
+          }
+          for (int j = 0; ok && j < nmax; ++j) {
+            for (int t = 0; ok && t < kNT; ++t) {
+              if (j >= n[t]) continue;
+              ok = next_kv();   // V
+              if (!ok) break;
+              ok = wait_all(bar_p_full(t, 0), p_count[t] & 1, kTagPFull);
+              if (!ok) break;
+              tc_fence_after_sync();
+              issue_pv(t, kv_count % C::kStages, j > 0, 0, kTileN / 32, bar_pv0_done(t));
+              ok = wait_all(bar_p_full(t, 1), p_count[t] & 1, kTagPFull);
+              if (!ok) break;
+              ++p_count[t];
+              tc_fence_after_sync();
+              issue_pv(t, kv_count % C::kStages, true, kTileN / 32, kTileN / 16, j == n[t] - 1 ? bar_o_full(t) : 0u);
+              umma_commit_elect(bar_kv_empty(kv_count % C::kStages));
+              ++kv_count;
+              if (j + 1 < n[t]) {
+                ok = next_kv();   // K of the next step
+                if (!ok) break;
+                issue_qk(t, kv_count % C::kStages, bar_s_full(t), q_release(t, j + 1), bar_kv_empty(kv_count % C::kStages));
+                ++kv_count;
+              }
+            }
+          }
+          if (!ok) break;
+          ++item_count;
+          continue;
+        }
         for (int t = 0; ok && t < kNT; ++t)
           ok = wait_all(bar_q_full(t), item_count & 1, kTagQFull);
         if (!ok) break;
@@ -440,6 +567,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
     const float scale_log2 = p.sm_scale * kLog2e;
     const float headroom = kHeadroomLog2 / scale_log2;   // in raw score units (sm_scale > 0 on this path)
     uint32_t item_count = 0, s_count = 0, o_count = 0;
+    uint32_t o1_count = 0;   // kSplitKeys: phases of o_full(1); o_count counts those of o_full(0) there
     bool ok = true;
 #ifdef RSFA_TRACE
     unsigned long long* trace_buf = (p.trace != nullptr && blockIdx.x == 0 && lane == 0)
@@ -455,12 +583,11 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
       if (item >= sched.total_items) break;
       ++item_count;
-      int bh, row0;
-      decode(item, bh, row0);
-      const int tile_row0 = row0 + t * kTileM;
+      int bh, tile_row0;
+      decode(item, t, bh, tile_row0);
       const int row = tile_row0 + row_in_tile;
-      const int n_tiles = num_kv_tiles(tile_row0, S, p.causal);
-      if (n_tiles == 0) continue;
+      const int n_tiles = tile_steps(t, bh, tile_row0);
+      if (kMode != kSplitKeys && n_tiles == 0) continue;
 
       // The reference maximum m_used of a row is set from the first key tile (plus headroom) and is
       // NOT recomputed per tile: a tile is exponentiated against the current reference straight
@@ -470,6 +597,9 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       // handles the remaining key tiles with a row maximum per half.  This replaces the per-tile
       // maximum of the reference's loop (:196-203) and its "rescale only when the maximum moved"
       // (:466-487) by "rescale only when it must".
+      auto wait_o_read = [&]() -> bool {
+        return item_count == 1 || mbar_wait_warp(bar_o_read, item_count & 1, abort_flag, wait_ns, kTagOFull);
+      };
       float m_used = -INFINITY;  // reference, in raw score units
       float l = 0.f;
       int j = 0;
@@ -495,7 +625,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         RSFA_TRACE_EV(0x2000 + j);   // S in registers
 
         // masked tile: the one crossing the diagonal, or the ragged end of the sequence
-        const int n0 = j * kTileN;
+        const int n0 = key_tile(t, j) * kTileN;
         const bool masked = (n0 + kTileN > S) || (p.causal && n0 + kTileN > tile_row0 + 1);
         if (masked) {
           int limit = S - 1 - n0;                           // last visible column of this tile
@@ -527,6 +657,11 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           float mb = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7]));
           if (mb == -INFINITY) mb = 0.f;  // only rows past S can get here; keep them finite
           m_used = mb + headroom;
+          if constexpr (kMode == kSplitKeys) {
+            // the first PV of an item overwrites O_t: both groups must have read the last item's
+            ok = wait_o_read();
+            if (!ok) break;
+          }
         }
         RSFA_TRACE_EV(0x3000 + j);   // reference ready
         const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
@@ -600,7 +735,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         // go back to the fast loop.  The PV MMAs of the tile's first half accumulate into O_t, so
         // the second half waits for them before it may rescale O_t.
         RSFA_TRACE_EV(0xc000 + j);
-        const int n0 = j * kTileN;
+        const int n0 = key_tile(t, j) * kTileN;
         int limit = S - 1 - n0;                             // last visible column of this tile
         if (p.causal) limit = min(limit, row - n0);
         for (int half = careful_half; half < 2; ++half) {
@@ -623,6 +758,42 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       }
       }
       if (!ok) break;
+
+      if constexpr (kMode == kSplitKeys) {
+        // ---- epilogue of two partial results.  Row r of both is in TMEM lane r, so a warp reads O_0 and O_1
+        // of its rows alike: group t merges and stores the columns [t * D / 2, (t + 1) * D / 2).  A tile that
+        // had no key tile (its l is zero) left nothing in O_t, which is then not looked at.
+        // a tile without steps has not waited yet: the last item's (m, l) may still be in use
+        if (n_tiles == 0) ok = wait_o_read();
+        if (!ok) break;
+        s_ml[t * kTileM + row_in_tile].x = m_used;
+        s_ml[t * kTileM + row_in_tile].y = l;
+        mbar_arrive(bar_ml_ready);
+        ok = mbar_wait_warp(bar_ml_ready, (item_count - 1) & 1, abort_flag, wait_ns, kTagOFull);
+        if (!ok) break;
+        const bool both = tile_steps(1, bh, tile_row0) > 0;
+        ok = mbar_wait_warp(bar_o_full(0), o_count & 1, abort_flag, wait_ns, kTagOFull);
+        if (ok && both) ok = mbar_wait_warp(bar_o_full(1), o1_count & 1, abort_flag, wait_ns, kTagOFull);
+        if (!ok) break;
+        ++o_count;
+        if (both) ++o1_count;
+        tc_fence_after_sync();
+        const float m0 = s_ml[row_in_tile].x, l0 = s_ml[row_in_tile].y;
+        const float m1 = s_ml[kTileM + row_in_tile].x, l1 = s_ml[kTileM + row_in_tile].y;
+        const float m = both ? fmaxf(m0, m1) : m0;
+        const float e0 = ex2((m0 - m) * scale_log2), e1 = both ? ex2((m1 - m) * scale_log2) : 0.f;
+        const float l_all = both ? l0 * e0 + l1 * e1 : l0;
+        const float inv_l = 1.f / l_all;
+        const int b = bh / p.H, h = bh - b * p.H;
+        const int wq = warp & 3;
+        const uint32_t tO0 = tmem_base + lane_base + C::kColO(0) + t * (D / 2);
+        const uint32_t tO1 = tmem_base + lane_base + C::kColO(1) + t * (D / 2);
+        merge_store_o_rows<D / 2, kBf16>(tO0, tO1, both, e0 * inv_l, e1 * inv_l, sStage + t * C::kStageBytes + wq * 4096, lane,
+                                         &maps.o, t * (D / 2), tile_row0 + wq * 32, h, b, tile_row0 + wq * 32 < S, bar_o_read);
+        if (t == 0 && p.lse != nullptr && row < S)
+          p.lse[static_cast<int64_t>(bh) * S + row] = m * p.sm_scale + logf(l_all);
+        continue;
+      }
 
       // ---- epilogue: O_t / l -> global, lse = m + log l
       ok = mbar_wait_warp(bar_o_full(t), o_count & 1, abort_flag, wait_ns, kTagOFull);
@@ -663,23 +834,24 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   }
 }
 
-template <int D, bool kBf16>
+template <int D, bool kBf16, int kMode>
 cudaError_t launch_one(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
-  using C = Cfg<D>;
+  using C = Cfg<D, kMode>;
   TmaMaps maps;
   if (!make_map(&maps.q, p.q, p, p.q_stride, kTileM) || !make_map(&maps.k, p.k, p, p.k_stride, kTileN) ||
       !make_map(&maps.v, p.v, p, p.v_stride, kTileN) || !make_map(&maps.o, p.o, p, p.o_stride, 32))
     return cudaErrorInvalidValue;
   SchedInfo sched;
-  sched.items_per_head = (p.S + kNT * kTileM - 1) / (kNT * kTileM);
-  sched.total_items = sched.items_per_head * p.B * p.H;
-  auto kern = fwd_tcgen05_kernel<D, kBf16>;
+  const int rows = kMode == kSplitKeys ? kTileM : kNT * kTileM;
+  sched.items_per_head = (p.S + rows - 1) / rows;
+  sched.total_items = kMode == kTwoHeads ? (p.B * p.H + kNT - 1) / kNT : sched.items_per_head * p.B * p.H;
+  auto kern = fwd_tcgen05_kernel<D, kBf16, kMode>;
   static std::atomic<unsigned long long> smem_done{0};   // per kernel instantiation, bit per device
   cudaError_t e = set_dynamic_smem_once(smem_done, reinterpret_cast<const void*>(kern), C::kSmemBytes);
   if (e != cudaSuccess) return e;
   // No memset of the work queue: the last CTA of the launch that used it before put it back to zero.
   const int grid = sched.total_items < sm_count ? sched.total_items : sm_count;
-  sched_set_tail(sched, p.B * p.H, p.causal, grid);
+  sched_set_tail(sched, p.B * p.H, kMode == kTwoHeads ? 0 : p.causal, grid);
   e = launch_persistent(kern, grid, kNumThreads, C::kSmemBytes, stream, p.pdl != 0, maps, p, sched);
   if (e == cudaSuccess) *launches += 1;
   return e;
@@ -728,18 +900,54 @@ void tcgen05_resolve_tile(int S, int D, int causal, int req_bm, int req_bn, int 
   }
 }
 
+namespace {
+template <int D, int kMode>
+cudaError_t launch_type(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
+  return p.bf16 ? launch_one<D, true, kMode>(p, sm_count, stream, launches)
+                : launch_one<D, false, kMode>(p, sm_count, stream, launches);
+}
+
+// Whether a D = 128 launch ends sooner with kSplitKeys items (128 rows, the two Q tiles of a CTA share the
+// keys) than with pairs of Q tiles (256 rows).  A pair step - both Q tiles x 128 keys - takes as long either
+// way, but twice as many items of half the length fill a GPU that has fewer pairs than multiprocessors, and
+// waste less of a last wave.  The times are fits to launches of 1 to 600 pairs, S = 256 ... 8192, in 10 ns:
+// 170 n + 200 for a pair item of n key tiles, 92 n + 220 for a split one (its steps load twice the K/V
+// bytes).  Without the mask all items are equal and come in waves; with it they come heaviest first, so a
+// launch takes the heaviest item or, if that is longer, its share of all of them (the 15 % and 1.5 us are for
+// the uneven end).  Measured, pairs -> split: 8 heads of S = 2048 34.1 -> 22.7 us, 2 of S = 8192 106 -> 59.5,
+// causal 99.6 -> 56.4; 25 heads of S = 2048 (1.35 waves of pairs) 57.8 -> 52.6; where it is not chosen it
+// would have cost 5 to 30 %.
+bool split_keys_pays(const FwdParams& p, int sm_count) {
+  const long long heads = static_cast<long long>(p.B) * p.H;
+  const long long n = (p.S + kTileN - 1) / kTileN;   // key tiles of a row, and blocks of 128 rows of a head
+  if (n < 2 || heads * n > 16ll * sm_count) return false;
+  const long long pairs = heads * ((n + 1) / 2);
+  const long long pair_item = 170 * n + 200, split_item = 92 * n + 220;
+  if (p.causal) {
+    const long long all = heads * (92 * n * (n + 1) / 2 + 220 * n);
+    const long long share = all * 115 / 100 / sm_count + 150;
+    return (split_item > share ? split_item : share) < pair_item;
+  }
+  const long long pair_waves = (pairs + sm_count - 1) / sm_count, split_waves = (heads * n + sm_count - 1) / sm_count;
+  return 100 * split_waves * split_item < 97 * pair_waves * pair_item;
+}
+}  // namespace
+
 cudaError_t launch_fwd_tcgen05(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
+  if (p.D == 128 && p.variant < 0) {
+    if (p.S <= kTileN && static_cast<long long>(p.B) * p.H > sm_count)
+      return launch_type<128, kTwoHeads>(p, sm_count, stream, launches);
+    if (split_keys_pays(p, sm_count)) return launch_type<128, kSplitKeys>(p, sm_count, stream, launches);
+  }
   // D = 256 exists only in the double-buffered family (its accumulator leaves room for one Q tile).
   if (p.tile_n == 64 || p.D == 256) return launch_fwd_tcgen05_db(p, sm_count, stream, launches);
-  if (p.D == 128) return p.bf16 ? launch_one<128, true>(p, sm_count, stream, launches)
-                                : launch_one<128, false>(p, sm_count, stream, launches);
+  if (p.D == 128) return launch_type<128, kPair>(p, sm_count, stream, launches);
   if (p.D <= 64) {
     // D = 64 (and below): the separate-P kernel, unless single-buffered S is forced.  A single key
     // tile (S <= 128) leaves nothing to overlap: this file's kernel then.
     if (p.variant != 0 && (p.S > kTileN || p.variant == 2) && tcgen05_sp_fits(p))
       return launch_fwd_tcgen05_sp(p, sm_count, stream, launches);
-    return p.bf16 ? launch_one<64, true>(p, sm_count, stream, launches)
-                  : launch_one<64, false>(p, sm_count, stream, launches);
+    return launch_type<64, kPair>(p, sm_count, stream, launches);
   }
   return cudaErrorInvalidValue;
 }

@@ -279,6 +279,62 @@ __device__ __forceinline__ void store_o_rows(uint32_t t_o, float inv_l, uint32_t
   }
 }
 
+// Epilogue of one warp for a row kept in two parts (a softmax over two sets of keys): its 32 rows of
+// c0 * O_0 + c1 * O_1, kCols columns in tensor memory at `t_o0` and `t_o1`, to the columns from `col` on of
+// global memory, staged and stored like store_o_rows.  `both` = false: O_1 holds nothing and is not read.
+// Arrives at `bar_read` (every lane) once the warp has read its part of both.
+template <int kCols, bool kBf16>
+__device__ __forceinline__ void merge_store_o_rows(uint32_t t_o0, uint32_t t_o1, bool both, float c0, float c1,
+                                                   uint32_t stage, int lane, const CUtensorMap* map_o, int col,
+                                                   int row_first, int h, int b, bool any_row, uint32_t bar_read) {
+  static_assert(kCols == 64, "one staging buffer of 64 columns");
+  uint32_t a0[32], a1[32];
+  tmem_ld_x32(t_o0, a0);
+  tmem_ld_x32(t_o0 + 32, a1);
+  tmem_wait_ld();
+  reg_fence_x32(a0);
+  reg_fence_x32(a1);
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    a0[c] = __float_as_uint(__uint_as_float(a0[c]) * c0);
+    a1[c] = __float_as_uint(__uint_as_float(a1[c]) * c0);
+  }
+  if (both) {
+    uint32_t b0[32], b1[32];
+    tmem_ld_x32(t_o1, b0);
+    tmem_ld_x32(t_o1 + 32, b1);
+    tmem_wait_ld();
+    reg_fence_x32(b0);
+    reg_fence_x32(b1);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      a0[c] = __float_as_uint(fmaf(__uint_as_float(b0[c]), c1, __uint_as_float(a0[c])));
+      a1[c] = __float_as_uint(fmaf(__uint_as_float(b1[c]), c1, __uint_as_float(a1[c])));
+    }
+  }
+  tc_fence_before_sync();
+  mbar_arrive(bar_read);
+  const bool issuer = (lane == 0);
+  if (issuer) tma_store_wait_read_but<0>();   // the store that last read this staging buffer is done with it
+  __syncwarp();
+  const uint32_t row_addr = stage + lane * 128;
+  const uint32_t sw = static_cast<uint32_t>(lane & 7);
+  auto pair = [](uint32_t lo, uint32_t hi) { return pack2<kBf16>(__uint_as_float(lo), __uint_as_float(hi)); };
+#pragma unroll
+  for (int c = 0; c < 32; c += 8) {
+    st_shared_v4(row_addr + (((c >> 3) ^ sw) << 4), pair(a0[c], a0[c + 1]), pair(a0[c + 2], a0[c + 3]),
+                 pair(a0[c + 4], a0[c + 5]), pair(a0[c + 6], a0[c + 7]));
+    st_shared_v4(row_addr + ((((c >> 3) + 4) ^ sw) << 4), pair(a1[c], a1[c + 1]), pair(a1[c + 2], a1[c + 3]),
+                 pair(a1[c + 4], a1[c + 5]), pair(a1[c + 6], a1[c + 7]));
+  }
+  fence_proxy_async();
+  __syncwarp();
+  if (issuer && any_row) {
+    tma_store_4d(map_o, stage, col, row_first, h, b);
+    tma_store_commit();
+  }
+}
+
 // Register budgets per warpgroup after the common set-up of the 384-thread kernels (the launch
 // allocates 168 per thread): two softmax warpgroups and the warpgroup of the TMA / MMA warps.
 // setmaxnreg.inc can only take registers that another warpgroup of the same CTA has released with

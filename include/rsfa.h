@@ -63,7 +63,9 @@ extern "C" {
  *   sm_scale     multiplies q.k before the softmax (:84, :199).
  *   block_m/n    the reference's BLOCK_M / BLOCK_N.  Results do not depend on them; they are a
  *                request that is honoured when such a tile is instantiated and otherwise replaced
- *                by the table's choice (rsfa_get_tiling).  Must be positive.
+ *                by the table's choice (rsfa_get_tiling).  Must be positive.  At D = 128 launches too
+ *                small to fill the device, and sequences of one key tile, run on forms of the
+ *                (128, 128) kernel made for them whatever was asked for.
  *   dtype        RSFA_DTYPE_F16 or RSFA_DTYPE_BF16 (:698 tests one bf16 case).
  *   stream       a cudaStream_t (NULL = default stream).  The call is asynchronous like the
  *                reference's kernel launches; it does not synchronise.
@@ -144,7 +146,8 @@ RSFA_API int rsfa_select_path(int S, int D, int causal, float sm_scale, int bloc
 
 /*
  * Number of work items rsfa_fwd splits this problem into: (batch, head, block of query rows) units
- * that the persistent tcgen05 kernels hand out through their queue (256 rows each, 128 at D = 256),
+ * that the persistent tcgen05 kernels hand out through their queue (256 rows each, 128 at D = 256; the
+ * forms for small launches, see rsfa_fwd, deal out the same rows in other portions),
  * or the CTAs of the short-sequence kernel (64 rows each, all on grid.x, so the count may exceed
  * 65535).  Counterpart of NUM_BLOCKS = cdiv(N_CTX, BLOCK_M) * Z * H (:289-294).  Needs no device.
  */

@@ -1,0 +1,85 @@
+"""The two forms of the D = 128 kernel in which each Q tile of a CTA has K/V tiles of its own - two heads per
+work item (S <= 128), and the keys of one block of rows dealt out to both tiles - on a B200 against the fp32
+oracle, at the sizes where their bookkeeping can go wrong."""
+import math
+
+import pytest
+import torch
+
+from oracle.attention_ref import attention_fp32, make_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fa(cuda_device):
+    import ascend_rsfa.flash_attention_forward as mod
+
+    return mod
+
+
+def agree(fa, dev, q, k, v, causal, scale):
+    u = 2.0 ** -11 if q.dtype == torch.float16 else 2.0 ** -8
+    n0 = fa.launch_count()
+    o, lse = fa.attention_with_lse(q.to(dev), k.to(dev), v.to(dev), causal, scale)
+    torch.cuda.synchronize()
+    fa.device_status()
+    assert fa.launch_count() - n0 == 1
+    ref, lse_ref = attention_fp32(q, k, v, causal, scale, return_lse=True)
+    # a weight and a result are each rounded once to 16 bits; fp16 weights below 2^-14 of the tile's range
+    # (2^-8 of the row's largest) keep an absolute error of 2^-19 of it: 2^-19 * S in the worst sum
+    assert float((o.cpu().float() - ref).abs().max()) <= (2 * u + q.shape[2] * 2.0 ** -19) * float(v.float().abs().max())
+    assert torch.allclose(lse.cpu(), lse_ref, atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S", [129, 256, 257, 384, 385, 640, 1000, 2048])
+def test_split_keys(fa, cuda_device, S, causal):
+    # one to sixteen key tiles, odd numbers of them, a tile without any (the first causal block), ragged ends
+    for B, H, dtype in ((1, 1, torch.float16), (2, 3, torch.bfloat16)):
+        q, k, v = make_inputs(B, H, S, 128, seed=S, dtype=dtype)
+        agree(fa, cuda_device, q, k, v, causal, 1.0 / math.sqrt(128))
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_split_keys_with_several_items_per_cta(fa, cuda_device, causal):
+    # causal: more items than CTAs, light ones last; else a launch of 1.35 waves of pairs, three of split items
+    B, H, S = (1, 18, 1280) if causal else (1, 25, 2048)
+    q, k, v = make_inputs(B, H, S, 128, seed=7)
+    agree(fa, cuda_device, q, k, v, causal, 1.0 / math.sqrt(128))
+
+
+@pytest.mark.parametrize("order", ["growing", "falling"])
+def test_split_keys_when_the_two_halves_have_far_apart_maxima(fa, cuda_device, order):
+    # |k| grows or falls with the key index, every second key tile a hundred times smaller: references move,
+    # tiles are redone, and the merge weighs one half with next to nothing
+    g = torch.Generator().manual_seed(5)
+    S = 1024
+    ramp = torch.linspace(0.05, 2.0, S) if order == "growing" else torch.linspace(2.0, 0.05, S)
+    ramp = ramp * torch.where((torch.arange(S) // 128) % 2 == 0, 1.0, 0.01)
+    k = (torch.randn(1, 2, S, 128, generator=g).sign() * ramp.view(1, 1, S, 1)).half()
+    q = torch.randn(1, 2, S, 128, generator=g).sign().half()
+    v = torch.randn(1, 2, S, 128, generator=g).half()
+    for causal in (False, True):
+        agree(fa, cuda_device, q, k, v, causal, 1.0)
+
+
+def test_split_keys_keeps_a_nan_in_its_row(fa, cuda_device):
+    q, k, v = make_inputs(1, 2, 512, 128, seed=9)
+    q[0, 1, 300, 5] = float("nan")
+    o = fa.attention(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), False, 0.1, 128, 128).cpu().float()
+    ref = attention_fp32(q, k, v, False, 0.1)
+    assert bool(torch.isnan(o[0, 1, 300]).all()) and int(torch.isnan(o).any(-1).sum()) == 1
+    keep = ~torch.isnan(ref)
+    assert float((o - ref)[keep].abs().max()) < 5e-3
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S,heads", [(65, 149), (100, 301), (128, 300), (127, 597)])
+def test_two_heads_per_item(fa, cuda_device, S, heads, causal):
+    # odd numbers of heads: the last item has one; more items than CTAs
+    for dtype in (torch.float16, torch.bfloat16):
+        q, k, v = make_inputs(1, heads, S, 128, seed=S, dtype=dtype)
+        agree(fa, cuda_device, q, k, v, causal, 1.0 / math.sqrt(128))
+    q, k, v = make_inputs(heads // 7, 7, S, 128, seed=S + 1)
+    agree(fa, cuda_device, q, k, v, causal, 0.5)
