@@ -66,6 +66,9 @@ bool short_fits(int S, int D, float sm_scale);
 // The double-buffered-S family (D = 64, 128, 256), selected by launch_fwd_tcgen05.
 cudaError_t launch_fwd_tcgen05_db(const FwdParams& p, int sm_count, cudaStream_t stream,
                                   long long* launches);
+// Its form for D <= 64 with one Q tile per CTA, and whether a launch is better off with it.
+cudaError_t launch_fwd_tcgen05_db_single(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches);
+bool single_tiles_pay(const FwdParams& p, int sm_count);
 // The D = 64 kernel with P in tensor-memory columns of its own (fwd_tcgen05_sp.cu), selected by launch_fwd_tcgen05.
 cudaError_t launch_fwd_tcgen05_sp(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches);
 // Whether a problem's work items can be numbered in that kernel's scheduler ring (fewer than 2^27).

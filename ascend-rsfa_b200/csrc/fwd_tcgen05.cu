@@ -939,6 +939,8 @@ cudaError_t launch_fwd_tcgen05(const FwdParams& p, int sm_count, cudaStream_t st
       return launch_type<128, kTwoHeads>(p, sm_count, stream, launches);
     if (split_keys_pays(p, sm_count)) return launch_type<128, kSplitKeys>(p, sm_count, stream, launches);
   }
+  if (p.D <= 64 && p.variant < 0 && p.S > kTileN && single_tiles_pay(p, sm_count))
+    return launch_fwd_tcgen05_db_single(p, sm_count, stream, launches);
   // D = 256 exists only in the double-buffered family (its accumulator leaves room for one Q tile).
   if (p.tile_n == 64 || p.D == 256) return launch_fwd_tcgen05_db(p, sm_count, stream, launches);
   if (p.D == 128) return launch_type<128, kPair>(p, sm_count, stream, launches);

@@ -17,7 +17,9 @@
 // even when it is already satisfied and a tcgen05.mma about 40, so one warp cannot feed both tiles.
 // TMEM columns: S_t[b] at 128 t + 64 b, O_t at 128 kNT + D t (kNT = 2 for D <= 128, 1 for D = 256).
 // Shared memory: Q tiles + a ring of K/V tiles of 64 keys filled by TMA (128-byte swizzle).
-// Roles: warps [0, 4 kNT) softmax (one thread per row), then one TMA warp and kNT MMA warps.
+// Roles: warps [0, 4 kNT) softmax (one thread per row), then one TMA warp, kNT MMA warps and, at D <= 128, one
+// warp that loads the Q tiles.
+// At D <= 64 there is also a form with one Q tile per CTA and two CTAs per SM (see single_tiles_pay).
 // D = 256 differs in three ways (see DbCfg): Q travels through the K/V ring and is copied into the
 // 128 spare tensor-memory columns by the MMA warp (tcgen05.cp), QK^T reads it from there (A in
 // tensor memory, only K from shared memory), and warps 8-11 do the epilogue so that the single
@@ -42,20 +44,28 @@ struct DbCfg {
   // A ring slot holds a PAIR of tiles that the MMA warps consume together: (K_0, K_1) first,
   // then (V_j, K_{j+2}) for j = 0, 1, ... - one full/empty barrier pair per slot.
   static constexpr int kSlotBytes = 2 * kKvBytes;
-  static constexpr int kStages = (D == 256) ? 3 : (D == 128 ? 4 : 6);
+  // One Q tile at D <= 64 needs half of everything (192 tensor-memory columns, 97 KB): two CTAs per SM.
+  static constexpr int kCtasPerSm = (NT == 1 && D != 256) ? 2 : 1;
+  static constexpr int kTmemCols = 512 / kCtasPerSm;
+  static constexpr int kStages = (D == 256) ? 3 : (kCtasPerSm == 2 ? 4 : (D == 128 ? 4 : 6));
   // D = 256 has a warpgroup of its own for the epilogue (warps 8-11; a warp reads the tensor-memory
   // lanes 32 * (warp % 4) ...): the single softmax group goes straight on to the next work item and
   // the O store runs beside that item's first key tiles.  Warps 6 and 7 have no role.
   static constexpr bool kEpi = (D == 256);
   static constexpr int kEpiWarp0 = 8;
-  static constexpr int kThreads = kEpi ? 384 : 32 * (4 * NT + 1 + NT);
+  // D <= 128: a warp of its own loads the Q tiles of the next item as soon as their buffers are free (behind
+  // the K/V tiles in the producer's order they were issued up to 4000 clk later)
+  static constexpr bool kQWarp = (D != 256);
+  static constexpr int kThreads = kEpi ? 384 : 32 * (4 * NT + 1 + NT + 1);
   static constexpr int kTmaWarp = 4 * NT;
   static constexpr int kMmaWarp0 = 4 * NT + 1;   // one MMA warp per Q tile
+  static constexpr int kQLoadWarp = kMmaWarp0 + NT;
   // q_full, q_empty, pv_done, o_full per tile; s_full, p_full per (tile, buffer); ring; scheduler
   // epilogue staging: 128 rows x 64 columns, twice at D = 256 (four chunks per row; the shared
   // memory is there once Q has no buffer of its own)
   static constexpr int kStageBufs = (D == 256) ? 2 : 1;
   static constexpr int kStageBytes = kStageBufs * kRowsDb * 128;
+
   static constexpr int kNumBarriers = 4 * NT + 4 * NT + NT + 2 * kStages + 4 + 2;
   // D = 256 leaves 128 tensor-memory columns free: Q lives there as the A operand of QK^T.  Those
   // MMAs then read only K from shared memory (with both operands there, N = 64 took 65 clk instead
@@ -67,7 +77,7 @@ struct DbCfg {
   static constexpr int kQSmemBytes = kQTmem ? 0 : NT * kQTileBytes;
   __host__ __device__ static constexpr int col_q() { return 128 * NT + D * NT; }
   static_assert(!kQTmem || (NT == 1 && kQTileBytes == kSlotBytes), "Q travels through a ring slot");
-  static constexpr int kSmemBytes = kQSmemBytes + kStages * kSlotBytes + NT * kStageBytes + 1024 + kNumBarriers * 8 + 128 + 512;
+  static constexpr int kSmemBytes = kQSmemBytes + kStages * kSlotBytes + NT * kStageBytes + 1024 + kNumBarriers * 8 + 144 + (kEpi ? 512 : 0);
   __host__ __device__ static constexpr int col_s(int t, int b) { return 128 * t + 64 * b; }
   __host__ __device__ static constexpr int col_o(int t) { return 128 * NT + D * t; }
 };
@@ -79,10 +89,10 @@ __device__ __forceinline__ int num_kv_tiles_db(int row0, int S, int causal) {
 }
 
 template <int D, int NT, bool kBf16>
-__global__ void __launch_bounds__(DbCfg<D, NT>::kThreads, 1)
+__global__ void __launch_bounds__(DbCfg<D, NT>::kThreads, DbCfg<D, NT>::kCtasPerSm)
 fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, const SchedInfo sched) {
   using C = DbCfg<D, NT>;
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = smem_base;
   const uint32_t sKV = sQ + C::kQSmemBytes;
@@ -102,11 +112,11 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
   // warp and softmax group (O has been read, s_inv_l may be written again)
   const uint32_t bar_epi_ready = bar_sched_empty0 + 16u;
   const uint32_t bar_o_free = bar_epi_ready + 8u;
-  const uint32_t misc = sBar + 8u * C::kNumBarriers;
+  const uint32_t misc = (sBar + 8u * C::kNumBarriers + 15u) & ~15u;
   uint8_t* misc_ptr = smem_raw + (misc - smem_u32(smem_raw));
   volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(misc_ptr);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc_ptr + 4);
-  volatile int* sched_ring = reinterpret_cast<volatile int*>(misc_ptr + 8);
+  const uint32_t sched_ring = misc + 16u;   // 2 slots of a WorkItem
   volatile float* s_inv_l = reinterpret_cast<volatile float*>(misc_ptr + 128);   // kRowsDb values
 
   const int warp = threadIdx.x >> 5;
@@ -131,8 +141,8 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_sched_full0 + 8u * s, 1);
-      // one lane per MMA warp, per softmax warp and per epilogue warp
-      mbar_init(bar_sched_empty0 + 8u * s, NT + 4 * NT + (C::kEpi ? 4 : 0));
+      // one lane per MMA warp, per softmax warp, per epilogue warp and of the Q loader
+      mbar_init(bar_sched_empty0 + 8u * s, NT + 4 * NT + (C::kEpi ? 4 : 0) + (C::kQWarp ? 1 : 0));
     }
     mbar_init(bar_epi_ready, kRowsDb);
     mbar_init(bar_o_free, 4);
@@ -140,7 +150,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
     fence_proxy_async();
   }
   if (warp == C::kMmaWarp0) {
-    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_base_slot)), 512);
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_base_slot)), C::kTmemCols);
     tmem_relinquish();
   }
   if (warp == C::kTmaWarp && lane == 0) {
@@ -157,55 +167,64 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
   griddep_wait();
 
   const int S = p.S;
-  auto decode = [&](int item, int& bh, int& row0) {
-    int blk;
-    sched_decode(sched, p.causal, item, bh, blk);
-    row0 = blk * (NT * kRowsDb);
-  };
-
   if (warp == C::kTmaWarp) {
     // ================================================================ producer
     if (lane == 0) {
       RSFA_TRACE_DECL(3);
-      uint32_t kv_count = 0, item_count = 0;
+      uint32_t kv_count = 0;
+      uint32_t claim_count = 0;    // work items claimed / published so far
+      uint32_t publish_count = 0;
       bool ok = true;
-      // D = 256: Q reaches the softmax warps through the ring, and at a work-item boundary everything
-      // waits for it (2 us from HBM).  So the Q tile of the NEXT item is sent on its way to L2 as early as
-      // the item is known: without the causal mask the next item is claimed while this one starts (all
-      // items take equally long, claiming one ahead costs no balance); with it, when it is claimed
-      // anyway, which is still two key tiles before its load can be issued.
-      int claimed = -1;
-      auto prefetch_q = [&](int it) {
-        if (it >= sched.total_items) return;
-        int pbh, prow0;
-        decode(it, pbh, prow0);
-        const int pb = pbh / p.H, ph = pbh - pb * p.H;
-        for (int bx = 0; bx < C::kBoxes; ++bx) tma_prefetch_l2_4d(&maps.q, bx * 64, prow0, ph, pb);
-      };
-      while (ok) {
-        const int slot = item_count & 1;
-        ok = mbar_wait(bar_sched_empty0 + 8u * slot, ((item_count >> 1) & 1) ^ 1, abort_flag, wait_ns, kTagSched);
-        if (!ok) break;
-        int item = claimed;
-        claimed = -1;
-        if (item < 0) {
-          // the first item of a CTA is its own index (grid <= number of items), the queue hands out the rest
-          item = (item_count == 0) ? static_cast<int>(blockIdx.x)
-                                   : static_cast<int>(atomicAdd(p.tile_counter, 1u) + gridDim.x);
-          if (C::kQTmem) prefetch_q(item);
+      // The next work item.  The first one of a CTA is its own index (grid <= number of items), the queue hands
+      // out the rest.
+      auto claim = [&]() -> WorkItem {
+        WorkItem w;
+        w.item = (claim_count++ == 0) ? static_cast<int>(blockIdx.x)
+                                      : static_cast<int>(atomicAdd(p.tile_counter, 1u) + gridDim.x);
+        w.b = w.h = w.row0 = 0;
+        if (w.item < sched.total_items) {
+          int bh, blk;
+          sched_decode(sched, p.causal, w.item, bh, blk);
+          w.b = bh / p.H;
+          w.h = bh - w.b * p.H;
+          w.row0 = blk * (NT * kRowsDb);
+          if constexpr (C::kQTmem) {
+            // D = 256: Q reaches the softmax warps through the ring, and at a work-item boundary everything waits
+            // for it (2 us from HBM), so it is sent on its way to L2 as early as the item is known.
+            for (int bx = 0; bx < C::kBoxes; ++bx) tma_prefetch_l2_4d(&maps.q, bx * 64, w.row0, w.h, w.b);
+          }
         }
-        sched_ring[slot] = item;
+        return w;
+      };
+      auto publish = [&](const WorkItem& w) -> bool {
+        const int slot = publish_count & 1;
+        if (!mbar_wait(bar_sched_empty0 + 8u * slot, ((publish_count >> 1) & 1) ^ 1, abort_flag, wait_ns, kTagSched))
+          return false;
+        ++publish_count;
+        ring_put(sched_ring + 16u * slot, w);
         __threadfence_block();
         mbar_arrive(bar_sched_full0 + 8u * slot);
-        if (item >= sched.total_items) {
-          griddep_launch_dependents();   // the queue is empty: the next kernel on the stream may set up
-          break;
-        }
-        int bh, row0;
-        decode(item, bh, row0);
-        const int b = bh / p.H, h = bh - b * p.H;
+        if (w.item >= sched.total_items) griddep_launch_dependents();   // the queue is empty: the next kernel may set up
+        return true;
+      };
+      WorkItem next = claim();
+      ok = publish(next);
+      while (ok && next.item < sched.total_items) {
+        const WorkItem cur = next;
+        const int b = cur.b, h = cur.h, row0 = cur.row0;
         int nmax = 0;
         for (int t = 0; t < NT; ++t) nmax = max(nmax, num_kv_tiles_db(row0 + t * kRowsDb, S, p.causal));
+        // The next item is claimed and published a few key tiles before the loads of this one end: the other
+        // roles then find it without waiting for the queue, and its Q is loaded as soon as there is room (with
+        // the WorkItem ring 1 to 4 % at D = 256, S = 1024 causal 330 -> 322 us, and 1 to 4 % at D <= 128).  Not
+        // earlier: a CTA that claims far ahead of its need unbalances the end of the launch.  (D = 256 without
+        // the mask: items all take equally long, and their Q is worth a whole item's head start.)
+        const int j_next = max(0, nmax - 4);
+        bool claimed = false;
+        if (C::kQTmem && !p.causal) {
+          next = claim();
+          claimed = true;
+        }
         // one ring entry: tile A (K_0 or V_j) and, when it exists, tile B (K_1 or K_{j+2})
         auto load_pair = [&](const CUtensorMap* map_a, int ja, bool has_b, int jb) -> bool {
           const uint32_t s = kv_count % C::kStages;
@@ -224,10 +243,6 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
           return true;
         };
         if constexpr (C::kQTmem) {
-          if (!p.causal) {
-            claimed = static_cast<int>(atomicAdd(p.tile_counter, 1u) + gridDim.x);
-            prefetch_q(claimed);
-          }
           // Q is the first ring entry of the item
           const uint32_t s = kv_count % C::kStages;
           const uint32_t ph = (kv_count / C::kStages) & 1;
@@ -239,19 +254,37 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
             tma_load_4d(sKV + s * C::kSlotBytes + bx * C::kQBoxBytes, &maps.q, bar_kv_full(s), bx * 64, row0, h, b);
           ++kv_count;
         }
-        // (K_0, K_1) before the Q tiles: ring slots free up while the previous item drains,
-        // whereas a Q buffer is released only when that item's last QK^T on it has finished.
         ok = load_pair(&maps.k, 0, nmax > 1, 1);
-        for (int t = 0; !C::kQTmem && ok && t < NT; ++t) {
+        for (int j = 0; ok && j < nmax; ++j) {
+          if (j == j_next) {
+            if (!claimed) next = claim();
+            ok = publish(next);
+            if (!ok) break;
+          }
+          ok = load_pair(&maps.v, j, j + 2 < nmax, j + 2);
+        }
+      }
+    }
+  } else if (C::kQWarp && warp == C::kQLoadWarp) {
+    // ================================================================ Q loader (D <= 128)
+    if (lane == 0) {
+      uint32_t item_count = 0;
+      bool ok = true;
+      while (ok) {
+        const int slot = item_count & 1;
+        ok = mbar_wait(bar_sched_full0 + 8u * slot, (item_count >> 1) & 1, abort_flag, wait_ns, kTagSched);
+        if (!ok) break;
+        const WorkItem w = ring_get(sched_ring + 16u * slot);
+        mbar_arrive(bar_sched_empty0 + 8u * slot);
+        if (w.item >= sched.total_items) break;
+        for (int t = 0; ok && t < NT; ++t) {
           ok = mbar_wait(bar_q_empty(t), (item_count & 1) ^ 1, abort_flag, wait_ns, kTagQEmpty);
           if (!ok) break;
-          RSFA_TRACE_EV(0x100 + t);
           mbar_arrive_expect_tx(bar_q_full(t), C::kQTileBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
-            tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64,
-                        row0 + t * kRowsDb, h, b);
+            tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64, w.row0 + t * kRowsDb,
+                        w.h, w.b);
         }
-        for (int j = 0; ok && j < nmax; ++j) ok = load_pair(&maps.v, j, j + 2 < nmax, j + 2);
         ++item_count;
       }
     }
@@ -282,12 +315,11 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       const int slot = item_count & 1;
       ok = wait_all(bar_sched_full0 + 8u * slot, (item_count >> 1) & 1, kTagSched);
       if (!ok) break;
-      const int item = __shfl_sync(0xffffffffu, sched_ring[slot], 0);
-      __syncwarp();
+      const WorkItem w = ring_get(sched_ring + 16u * slot);
+      const int item = __shfl_sync(0xffffffffu, w.item, 0);
+      const int row0 = __shfl_sync(0xffffffffu, w.row0, 0);
       if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
       if (item >= sched.total_items) break;
-      int bh, row0;
-      decode(item, bh, row0);
       int nmax = 0;
       for (int tt = 0; tt < NT; ++tt) nmax = max(nmax, num_kv_tiles_db(row0 + tt * kRowsDb, S, p.causal));
       const int n = num_kv_tiles_db(row0 + t * kRowsDb, S, p.causal);
@@ -420,14 +452,12 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       const int slot = item_count & 1;
       ok = mbar_wait_warp(bar_sched_full0 + 8u * slot, (item_count >> 1) & 1, abort_flag, wait_ns, kTagSched);
       if (!ok) break;
-      const int item = sched_ring[slot];
+      const WorkItem w = ring_get(sched_ring + 16u * slot);
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
-      if (item >= sched.total_items) break;
+      if (w.item >= sched.total_items) break;
       ++item_count;
-      int bh, row0;
-      decode(item, bh, row0);
-      const int tile_row0 = row0 + t * kRowsDb;
+      const int tile_row0 = w.row0 + t * kRowsDb;
       const int row = tile_row0 + row_in_tile;
       const int n = num_kv_tiles_db(tile_row0, S, p.causal);
       if (n == 0) continue;
@@ -556,7 +586,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         s_inv_l[row_in_tile] = 1.f / l;
         mbar_arrive(bar_epi_ready);
         if (p.lse != nullptr && row < S)
-          p.lse[static_cast<int64_t>(bh) * S + row] = m_used * p.sm_scale + logf(l);
+          p.lse[(static_cast<int64_t>(w.b) * p.H + w.h) * S + row] = m_used * p.sm_scale + logf(l);
         RSFA_TRACE_EV(0x7000);   // item handed to the epilogue warps
       }
       if constexpr (C::kEpi) continue;
@@ -567,7 +597,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       tc_fence_after_sync();
       RSFA_TRACE_EV(0x6000);   // O seen
       const float inv_l = 1.f / l;
-      const int b = bh / p.H, h = bh - b * p.H;
+      const int b = w.b, h = w.h;
       // O_t / l -> global memory: each warp stages and stores its own 32 rows (store_o_rows)
       {
         const int wq = warp & 3;
@@ -575,7 +605,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
                                               &maps.o, tile_row0 + wq * 32, h, b, tile_row0 + wq * 32 < S);
       }
       if (p.lse != nullptr && row < S)
-        p.lse[static_cast<int64_t>(bh) * S + row] = m_used * p.sm_scale + logf(l);
+        p.lse[(static_cast<int64_t>(w.b) * p.H + w.h) * S + row] = m_used * p.sm_scale + logf(l);
       tc_fence_before_sync();
       RSFA_TRACE_EV(0x7000);   // epilogue done
     }
@@ -596,13 +626,11 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       const int slot = item_count & 1;
       ok = mbar_wait_warp(bar_sched_full0 + 8u * slot, (item_count >> 1) & 1, abort_flag, wait_ns, kTagSched);
       if (!ok) break;
-      const int item = sched_ring[slot];
+      const WorkItem w = ring_get(sched_ring + 16u * slot);
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
-      if (item >= sched.total_items) break;
-      int bh, row0;
-      decode(item, bh, row0);
-      const int b = bh / p.H, h = bh - b * p.H;
+      if (w.item >= sched.total_items) break;
+      const int b = w.b, h = w.h, row0 = w.row0;
       ok = mbar_wait_warp(bar_epi_ready, item_count & 1, abort_flag, wait_ns, kTagOFull);
       if (!ok) break;
       const float inv_l = s_inv_l[wq * 32 + lane];
@@ -632,7 +660,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  if (warp == C::kMmaWarp0) tmem_dealloc(tmem_base, 512);
+  if (warp == C::kMmaWarp0) tmem_dealloc(tmem_base, C::kTmemCols);
   if (threadIdx.x == 0) {
     if (*abort_flag != 0) atomicCAS(p.status, 0, *abort_flag);
     queue_retire(p.tile_counter);
@@ -654,7 +682,8 @@ cudaError_t launch_db(const FwdParams& p, int sm_count, cudaStream_t stream, lon
   cudaError_t e = set_dynamic_smem_once(smem_done, reinterpret_cast<const void*>(kern), C::kSmemBytes);
   if (e != cudaSuccess) return e;
   // No memset of the work queue: the last CTA of the launch that used it before put it back to zero.
-  const int grid = sched.total_items < sm_count ? sched.total_items : sm_count;
+  const int slots = sm_count * C::kCtasPerSm;
+  const int grid = sched.total_items < slots ? sched.total_items : slots;
   sched_set_tail(sched, p.B * p.H, p.causal, grid);
   e = launch_persistent(kern, grid, C::kThreads, C::kSmemBytes, stream, p.pdl != 0, maps, p, sched);
   if (e == cudaSuccess) *launches += 1;
@@ -662,6 +691,29 @@ cudaError_t launch_db(const FwdParams& p, int sm_count, cudaStream_t stream, lon
 }
 
 }  // namespace
+
+// Whether a launch with D <= 64 ends sooner on this kernel with one Q tile per CTA and two CTAs per SM than on
+// the kernels whose CTAs own a pair of Q tiles.  Two CTAs that know nothing of each other hide each other's
+// work-item boundaries (last PV, epilogue, first QK^T: 3000 to 5000 clk, as long as two to three key tiles) and
+// deal out 128 rows at a time, where a pair ends when its longer tile does; but each loads its own K/V tiles and
+// a step is only 64 keys, so long rows in plenty are better off with the separate-P kernel (128 keys, K/V shared).
+// Measured at D = 64, best pair kernel -> this, us: S = 200 128 heads x 1000 / 128 36.5 -> 34.6, 300 heads 16.9 ->
+// 15.2; S = 384 1000 heads 75.2 -> 61.4, causal 59.0 -> 49.1; S = 512 causal 128 heads 15.3 -> 14.4, 1000 heads
+// 78.2 -> 74.6; S = 1024 causal 12 heads 17.0 -> 13.7, 1000 heads 229.6 -> 225.4; S = 2048 causal 12 heads 28.7 ->
+// 22.4, 48 heads 43.7 -> 42.8.  Beyond the lines drawn here it loses: S = 1024 300 heads 111 -> 115, S = 2048 167 ->
+// 180, causal S = 2048 128 heads 101.6 -> 104.2, S = 3000 40 heads 70.1 -> 70.9; causal S <= 160 (a second tile of a few rows) 25.8 -> 26.5, and causal
+// S <= 256 when pairs fill one wave but single tiles need second places on the SMs, 7.5 -> 8.2.
+bool single_tiles_pay(const FwdParams& p, int sm_count) {
+  const long long tiles = static_cast<long long>(p.B) * p.H * ((p.S + kRowsDb - 1) / kRowsDb);
+  if (!p.causal) return p.S <= 512 || (p.S <= 1024 && tiles <= 13ll * sm_count);
+  if (p.S <= 256 && tiles > sm_count) return p.S > 160 && tiles > 2 * sm_count;
+  return p.S <= 1024 || tiles <= 5ll * sm_count;
+}
+
+cudaError_t launch_fwd_tcgen05_db_single(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
+  if (p.D > 64) return cudaErrorInvalidValue;
+  return p.bf16 ? launch_db<64, 1, true>(p, sm_count, stream, launches) : launch_db<64, 1, false>(p, sm_count, stream, launches);
+}
 
 cudaError_t launch_fwd_tcgen05_db(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
   switch (p.D < 64 ? 64 : p.D) {

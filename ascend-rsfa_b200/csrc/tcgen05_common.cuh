@@ -102,6 +102,21 @@ __device__ __forceinline__ void sched_decode(const SchedInfo& sched, int causal,
   }
 }
 
+// A work item as the scheduler ring hands it to the roles of a CTA, taken apart once by the producer: the two
+// integer divisions are 300 clk that every role would otherwise spend at each work-item boundary.
+struct WorkItem {
+  int item;        // >= SchedInfo::total_items: no more work
+  int b, h, row0;  // batch, head, first row
+};
+__device__ __forceinline__ void ring_put(uint32_t slot_addr, const WorkItem& w) {
+  st_shared_v4(slot_addr, static_cast<uint32_t>(w.item), static_cast<uint32_t>(w.b), static_cast<uint32_t>(w.h),
+               static_cast<uint32_t>(w.row0));
+}
+__device__ __forceinline__ WorkItem ring_get(uint32_t slot_addr) {
+  const uint4 v = ld_shared_v4(slot_addr);
+  return {static_cast<int>(v.x), static_cast<int>(v.y), static_cast<int>(v.z), static_cast<int>(v.w)};
+}
+
 template <bool kBf16>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   if constexpr (kBf16) {

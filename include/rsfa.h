@@ -63,9 +63,9 @@ extern "C" {
  *   sm_scale     multiplies q.k before the softmax (:84, :199).
  *   block_m/n    the reference's BLOCK_M / BLOCK_N.  Results do not depend on them; they are a
  *                request that is honoured when such a tile is instantiated and otherwise replaced
- *                by the table's choice (rsfa_get_tiling).  Must be positive.  At D = 128 launches too
- *                small to fill the device, and sequences of one key tile, run on forms of the
- *                (128, 128) kernel made for them whatever was asked for.
+ *                by the table's choice (rsfa_get_tiling).  Must be positive.  Launches too small to
+ *                fill the device, sequences of one key tile and, at D <= 64, short and medium sequences
+ *                run on forms of the kernels made for them whatever was asked for.
  *   dtype        RSFA_DTYPE_F16 or RSFA_DTYPE_BF16 (:698 tests one bf16 case).
  *   stream       a cudaStream_t (NULL = default stream).  The call is asynchronous like the
  *                reference's kernel launches; it does not synchronise.

@@ -83,3 +83,26 @@ def test_two_heads_per_item(fa, cuda_device, S, heads, causal):
         agree(fa, cuda_device, q, k, v, causal, 1.0 / math.sqrt(128))
     q, k, v = make_inputs(heads // 7, 7, S, 128, seed=S + 1)
     agree(fa, cuda_device, q, k, v, causal, 0.5)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S", [129, 191, 256, 257, 320, 512, 513, 1000, 1024])
+def test_single_q_tiles_at_small_head_dimensions(fa, cuda_device, S, causal):
+    # one tile per CTA, two CTAs per SM: odd and even numbers of 64-key tiles, a last tile of one row, more items
+    # than places; D below 64 reads zero columns
+    for B, H, D, dtype in ((1, 1, 64, torch.float16), (2, 3, 32, torch.bfloat16), (1, 5, 16, torch.float16)):
+        q, k, v = make_inputs(B, H, S, D, seed=S + D, dtype=dtype)
+        agree(fa, cuda_device, q, k, v, causal, 1.0 / math.sqrt(D))
+    if S in (257, 512):
+        q, k, v = make_inputs(8, 33, S, 64, seed=S)
+        agree(fa, cuda_device, q, k, v, causal, 0.125)
+
+
+def test_single_q_tiles_follow_a_growing_maximum(fa, cuda_device):
+    g = torch.Generator().manual_seed(6)
+    S = 1024
+    k = (torch.randn(1, 2, S, 64, generator=g).sign() * torch.linspace(0.05, 3.0, S).view(1, 1, S, 1)).half()
+    q = torch.randn(1, 2, S, 64, generator=g).sign().half()
+    v = torch.randn(1, 2, S, 64, generator=g).half()
+    for causal in (False, True):
+        agree(fa, cuda_device, q, k, v, causal, 1.0)
