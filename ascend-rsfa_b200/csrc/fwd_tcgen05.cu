@@ -85,7 +85,7 @@ struct Cfg {
   static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4 + 2;
   static constexpr int kMlBytes = (kMode == kSplitKeys) ? kNT * kTileM * 8 : 0;   // (m, l) of every row, twice
   static constexpr int kSmemBytes = kQBufs * kQTileBytes + kStages * kKvTileBytes + kNT * kStageBytes + 1024 /*align*/ +
-                                    kNumBarriers * 8 + 64 + kMlBytes;
+                                    kNumBarriers * 8 + 80 + kMlBytes;
   __host__ __device__ static constexpr int kColS(int t) { return t * kTileN; }
   __host__ __device__ static constexpr int kColO(int t) { return 2 * kTileN + t * D; }
 };
@@ -124,12 +124,12 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   // kSplitKeys: (m, l) of both tiles are in shared memory / both groups have read O_0 and O_1
   const uint32_t bar_ml_ready = bar_sched_empty0 + 16u;
   const uint32_t bar_o_read = bar_ml_ready + 8u;
-  const uint32_t misc = sBar + 8u * C::kNumBarriers;
-  // misc words: [0] TMEM base, [1] abort flag, [2..3] scheduler ring, then for kSplitKeys (m, l) per row
+  const uint32_t misc = (sBar + 8u * C::kNumBarriers + 15u) & ~15u;
+  // misc: [0] TMEM base, [1] abort flag, from byte 16 on the scheduler ring, then for kSplitKeys (m, l) per row
   uint8_t* misc_ptr = smem_raw + (misc - smem_u32(smem_raw));
   volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(misc_ptr);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc_ptr + 4);
-  volatile int* sched_ring = reinterpret_cast<volatile int*>(misc_ptr + 8);
+  const uint32_t sched_ring = misc + 16u;   // 2 slots of a WorkItem
   volatile float2* s_ml = reinterpret_cast<volatile float2*>(misc_ptr + 64);   // [kNT][kTileM]
 
   const int warp = threadIdx.x >> 5;
@@ -180,23 +180,15 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   griddep_wait();
 
   const int S = p.S;
-  // work item -> (head, first row) of Q tile t.  Causal: heaviest (last) row block first.
-  auto decode = [&](int item, int t, int& bh, int& row0) {
-    if constexpr (kMode == kTwoHeads) {
-      bh = item * kNT + t;
-      row0 = 0;
-    } else {
-      int blk;
-      sched_decode(sched, p.causal, item, bh, blk);
-      row0 = kMode == kPair ? blk * (kNT * kTileM) + t * kTileM : blk * kTileM;
-    }
-  };
-  // number of key tiles of Q tile t (0: it has nothing to do in this item)
-  auto tile_steps = [&](int t, int bh, int row0) -> int {
-    if (kMode == kTwoHeads && bh >= p.B * p.H) return 0;
+  // number of key tiles of Q tile t, whose first row is row0 (0: it has nothing to do in this item; kTwoHeads:
+  // head t of the item, the last of which may have one only)
+  auto tile_steps = [&](int t, const WorkItem& w, int row0) -> int {
+    if (kMode == kTwoHeads && w.item * kNT + t >= p.B * p.H) return 0;
     const int n = num_kv_tiles(row0, S, p.causal);
     return kMode == kSplitKeys ? (n + 1 - t) / 2 : n;
   };
+  // first row of Q tile t of an item
+  auto tile_row = [](int t, const WorkItem& w) -> int { return kMode == kPair ? w.row0 + t * kTileM : w.row0; };
   // key tile of step j of Q tile t
   auto key_tile = [](int t, int j) -> int { return kMode == kSplitKeys ? 2 * j + t : j; };
 
@@ -221,12 +213,22 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         if (!ok) break;
         // The first item of a CTA is its own index (the grid is never larger than the number of items): no
         // round trip to the queue stands before the first loads.  The queue hands out the items behind those.
-        const int item = (item_count == 0) ? static_cast<int>(blockIdx.x)
-                                           : static_cast<int>(atomicAdd(p.tile_counter, 1u) + gridDim.x);
-        sched_ring[slot] = item;
+        WorkItem w;
+        w.item = (item_count == 0) ? static_cast<int>(blockIdx.x)
+                                   : static_cast<int>(atomicAdd(p.tile_counter, 1u) + gridDim.x);
+        w.b = w.h = w.row0 = 0;
+        if (w.item < sched.total_items) {
+          // causal: heaviest (last) row block first
+          int bh = w.item * kNT, blk = 0;
+          if constexpr (kMode != kTwoHeads) sched_decode(sched, p.causal, w.item, bh, blk);
+          w.b = bh / p.H;
+          w.h = bh - w.b * p.H;
+          w.row0 = blk * (kMode == kPair ? kNT * kTileM : kTileM);
+        }
+        ring_put(sched_ring + 16u * slot, w);
         __threadfence_block();
         mbar_arrive(bar_sched_full0 + 8u * slot);
-        if (item >= sched.total_items) {
+        if (w.item >= sched.total_items) {
           griddep_launch_dependents();   // the queue is empty: the next kernel on the stream may set up
           break;
         }
@@ -234,18 +236,14 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         int nmax = 0;
 #pragma unroll
         for (int t = 0; t < kNT; ++t) {
-          if (kMode == kPair && t > 0) {   // the same head, the next block of rows
-            tb[t] = tb[0];
-            th[t] = th[0];
-            trow[t] = trow[0] + t * kTileM;
-            n[t] = num_kv_tiles(trow[t], S, p.causal);
-          } else {
-            int bh;
-            decode(item, t, bh, trow[t]);
-            tb[t] = bh / p.H;
-            th[t] = bh - tb[t] * p.H;
-            n[t] = tile_steps(t, bh, trow[t]);
+          tb[t] = w.b;
+          th[t] = w.h;
+          if (kMode == kTwoHeads && t == 1 && ++th[t] == p.H) {
+            th[t] = 0;
+            ++tb[t];
           }
+          trow[t] = tile_row(t, w);
+          n[t] = tile_steps(t, w, trow[t]);
           nmax = max(nmax, n[t]);
         }
 
@@ -325,23 +323,17 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         const int slot = item_count & 1;
         ok = wait_all(bar_sched_full0 + 8u * slot, (item_count >> 1) & 1, kTagSched);
         if (!ok) break;
-        const int item = __shfl_sync(0xffffffffu, sched_ring[slot], 0);
-        __syncwarp();
+        WorkItem w = ring_get(sched_ring + 16u * slot);
+        w.item = __shfl_sync(0xffffffffu, w.item, 0);
+        w.row0 = __shfl_sync(0xffffffffu, w.row0, 0);
         if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
-        if (item >= sched.total_items) break;
+        if (w.item >= sched.total_items) break;
         RSFA_TRACE_EV(0xa000);   // item known
         int n[kNT];
         int nmax = 0;
-        int bh, row0;
-        decode(item, 0, bh, row0);
-        n[0] = tile_steps(0, bh, row0);
-        nmax = n[0];
 #pragma unroll
-        for (int t = 1; t < kNT; ++t) {
-          if (kMode == kPair)
-            n[t] = num_kv_tiles(row0 + t * kTileM, S, p.causal);
-          else
-            n[t] = tile_steps(t, kMode == kTwoHeads ? bh + t : bh, row0);
+        for (int t = 0; t < kNT; ++t) {
+          n[t] = tile_steps(t, w, tile_row(t, w));
           nmax = max(nmax, n[t]);
         }
         // S_t = Q_t K^T : both operands K-major, 64-column boxes, 8-row atoms of 1024 B.  A step
@@ -441,17 +433,18 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           ++item_count;
           continue;
         }
-        for (int t = 0; ok && t < kNT; ++t)
-          ok = wait_all(bar_q_full(t), item_count & 1, kTagQFull);
-        if (!ok) break;
-        RSFA_TRACE_EV(0xa100);   // Q present
         const uint32_t base = kv_count;  // K_j at base + 2j, V_j at base + 2j + 1
         if (nmax > 0) {
           ok = wait_kv(base);
           if (!ok) break;
-          tc_fence_after_sync();
           RSFA_TRACE_EV(0xa200);   // K_0 present
-          for (int t = 0; t < kNT; ++t) {
+          for (int t = 0; ok && t < kNT; ++t) {
+            // Each tile's first QK^T as soon as its own Q is there: Q_1 comes 1000 clk behind Q_0.  (This and the
+            // items taken apart by the producer: S = 200 37.8 -> 36.2 us, 16 x 8 heads of S = 2048 causal 139.3 ->
+            // 137.0, 64 heads of S = 128 6.65 -> 6.28.)
+            ok = wait_all(bar_q_full(t), item_count & 1, kTagQFull);
+            if (!ok) break;
+            tc_fence_after_sync();
             // Q_t is dead once its last QK^T MMA has run: release it so the next item's Q load
             // overlaps the rest of this item.
             if (n[t] > 0)
@@ -459,6 +452,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
             else
               umma_commit_elect(bar_q_empty(t));
           }
+          if (!ok) break;
           umma_commit_elect(bar_kv_empty(base % C::kStages));
         }
         // Steady state, kept free of everything the end of an item needs: while both tiles have key tiles
@@ -578,15 +572,14 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       const int slot = item_count & 1;
       ok = mbar_wait_warp(bar_sched_full0 + 8u * slot, (item_count >> 1) & 1, abort_flag, wait_ns, kTagSched);
       if (!ok) break;
-      const int item = sched_ring[slot];
+      const WorkItem w = ring_get(sched_ring + 16u * slot);
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_sched_empty0 + 8u * slot);
-      if (item >= sched.total_items) break;
+      if (w.item >= sched.total_items) break;
       ++item_count;
-      int bh, tile_row0;
-      decode(item, t, bh, tile_row0);
+      const int tile_row0 = tile_row(t, w);
       const int row = tile_row0 + row_in_tile;
-      const int n_tiles = tile_steps(t, bh, tile_row0);
+      const int n_tiles = tile_steps(t, w, tile_row0);
       if (kMode != kSplitKeys && n_tiles == 0) continue;
 
       // The reference maximum m_used of a row is set from the first key tile (plus headroom) and is
@@ -771,7 +764,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         mbar_arrive(bar_ml_ready);
         ok = mbar_wait_warp(bar_ml_ready, (item_count - 1) & 1, abort_flag, wait_ns, kTagOFull);
         if (!ok) break;
-        const bool both = tile_steps(1, bh, tile_row0) > 0;
+        const bool both = tile_steps(1, w, tile_row0) > 0;
         ok = mbar_wait_warp(bar_o_full(0), o_count & 1, abort_flag, wait_ns, kTagOFull);
         if (ok && both) ok = mbar_wait_warp(bar_o_full(1), o1_count & 1, abort_flag, wait_ns, kTagOFull);
         if (!ok) break;
@@ -784,14 +777,13 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         const float e0 = ex2((m0 - m) * scale_log2), e1 = both ? ex2((m1 - m) * scale_log2) : 0.f;
         const float l_all = both ? l0 * e0 + l1 * e1 : l0;
         const float inv_l = 1.f / l_all;
-        const int b = bh / p.H, h = bh - b * p.H;
         const int wq = warp & 3;
         const uint32_t tO0 = tmem_base + lane_base + C::kColO(0) + t * (D / 2);
         const uint32_t tO1 = tmem_base + lane_base + C::kColO(1) + t * (D / 2);
         merge_store_o_rows<D / 2, kBf16>(tO0, tO1, both, e0 * inv_l, e1 * inv_l, sStage + t * C::kStageBytes + wq * 4096, lane,
-                                         &maps.o, t * (D / 2), tile_row0 + wq * 32, h, b, tile_row0 + wq * 32 < S, bar_o_read);
+                                         &maps.o, t * (D / 2), tile_row0 + wq * 32, w.h, w.b, tile_row0 + wq * 32 < S, bar_o_read);
         if (t == 0 && p.lse != nullptr && row < S)
-          p.lse[static_cast<int64_t>(bh) * S + row] = m * p.sm_scale + logf(l_all);
+          p.lse[(static_cast<int64_t>(w.b) * p.H + w.h) * S + row] = m * p.sm_scale + logf(l_all);
         continue;
       }
 
@@ -802,7 +794,11 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       tc_fence_after_sync();
       RSFA_TRACE_EV(0x6000);         // O complete seen
       const float inv_l = 1.f / l;
-      const int b = bh / p.H, h = bh - b * p.H;
+      int b = w.b, h = w.h;
+      if (kMode == kTwoHeads && t == 1 && ++h == p.H) {
+        h = 0;
+        ++b;
+      }
       // O_t / l -> global memory: each warp stages and stores its own 32 rows (store_o_rows)
       {
         const int wq = warp & 3;
@@ -810,7 +806,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
                                tile_row0 + wq * 32 < S);
       }
       if (p.lse != nullptr && row < S)
-        p.lse[static_cast<int64_t>(bh) * S + row] = m_used * p.sm_scale + logf(l);
+        p.lse[(static_cast<int64_t>(b) * p.H + h) * S + row] = m_used * p.sm_scale + logf(l);
       tc_fence_before_sync();
       RSFA_TRACE_EV(0x7000);         // epilogue done
     }
