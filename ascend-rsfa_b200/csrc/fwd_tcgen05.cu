@@ -78,11 +78,11 @@ struct Cfg {
   static constexpr int kQTileBytes = kTileM * D * 2;
   static constexpr int kQBufs = (kMode == kSplitKeys) ? 1 : kNT;   // its two tiles have the same rows
   static constexpr int kKvTileBytes = kTileN * D * 2;
-  static constexpr int kStages = (D == 128) ? 4 : 6;
+  static constexpr int kStages = 4;
   static constexpr int kQBoxBytes = kTileM * 128;             // 128 rows x 128 B
   static constexpr int kKvBoxBytes = kTileN * 128;
   static constexpr int kStageBytes = kTileM * 128;            // epilogue staging: 128 rows x 64 columns
-  static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4 + 2;
+  static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4 + 2 + 2;
   static constexpr int kMlBytes = (kMode == kSplitKeys) ? kNT * kTileM * 8 : 0;   // (m, l) of every row, twice
   static constexpr int kSmemBytes = kQBufs * kQTileBytes + kStages * kKvTileBytes + kNT * kStageBytes + 1024 /*align*/ +
                                     kNumBarriers * 8 + 80 + kMlBytes;
@@ -114,8 +114,21 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   auto bar_kv_full = [&](int s) { return sBar + 8u * (2 * kNT + s); };
   auto bar_kv_empty = [&](int s) { return sBar + 8u * (2 * kNT + C::kStages + s); };
   auto bar_s_full = [&](int t) { return sBar + 8u * (2 * kNT + 2 * C::kStages + t); };
-  // P_t is handed to the MMA warp in two halves of 64 keys so the first PV MMAs start early.
-  auto bar_p_full = [&](int t, int half) { return sBar + 8u * (3 * kNT + 2 * C::kStages + 2 * t + half); };
+  // P_t is handed to the MMA warp in two halves of 64 keys so the first PV MMAs start early.  kPair: the MMA
+  // warp needs V_j with the first half of P_0(j) and K_{j+1} with the second, so the bytes of those loads are
+  // counted on the same barriers and one wait says both.  The loads run up to two steps ahead of the softmax:
+  // tile 0's barriers are two pairs used in turn (`step` = its key tiles so far).  Two waits per step less (four
+  // instead of six for the warp that paces the CTA): (16, 16, 4096, 128) causal 911 -> 894 us, (128, 8, 2048, 128)
+  // 1925 -> 1877, S = 1024 causal 86.6 -> 84.7.
+  const uint32_t bar_p0_odd = sBar + 8u * (C::kNumBarriers - 2);
+  auto bar_p_full = [&](int t, int half, uint32_t step) {
+    const uint32_t even = sBar + 8u * (3 * kNT + 2 * C::kStages + 2 * t + half);
+    return (kMode == kPair && t == 0 && (step & 1) != 0) ? bar_p0_odd + 8u * half : even;
+  };
+  auto p_parity = [](int t, uint32_t step) -> uint32_t { return (kMode == kPair && t == 0) ? (step >> 1) & 1 : step & 1; };
+  // kPair: what is not counted on those: K_0 of an item (two in turn), V_j of a step that only tile 1 has
+  auto bar_k_first = [&](uint32_t item_count) { return bar_kv_full(item_count & 1); };
+  const uint32_t bar_v_lone = bar_kv_full(2);
   auto bar_o_full = [&](int t) { return sBar + 8u * (5 * kNT + 2 * C::kStages + t); };
   // completion of the PV MMAs of a tile's first 64 keys (waited on only by the softmax slow path)
   auto bar_pv0_done = [&](int t) { return sBar + 8u * (7 * kNT + 2 * C::kStages + t); };
@@ -145,8 +158,10 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       mbar_init(bar_q_full(t), 1);
       mbar_init(bar_q_empty(t), 1);
       mbar_init(bar_s_full(t), 1);
-      mbar_init(bar_p_full(t, 0), kTileM);
-      mbar_init(bar_p_full(t, 1), kTileM);
+      for (uint32_t step = 0; step < (kMode == kPair && t == 0 ? 2u : 1u); ++step) {
+        mbar_init(bar_p_full(t, 0, step), kTileM + (kMode == kPair && t == 0 ? 1 : 0));
+        mbar_init(bar_p_full(t, 1, step), kTileM + (kMode == kPair && t == 0 ? 1 : 0));
+      }
       mbar_init(bar_o_full(t), 1);
       mbar_init(bar_pv0_done(t), 1);
     }
@@ -204,6 +219,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       RSFA_TRACE_DECL(3);
       uint32_t kv_count = 0;   // K/V tiles loaded so far (ring position)
       uint32_t item_count = 0; // work items started so far
+      uint32_t p0_steps = 0;   // kPair: key tiles of tile 0 so far
       bool ok = true;
       while (ok) {
         // fetch the next work item and publish it to the other roles
@@ -255,7 +271,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
             tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64, trow[t], th[t], tb[t]);
           return true;
         };
-        auto load_kv = [&](const CUtensorMap* map, int t, int j) -> bool {
+        auto load_kv = [&](const CUtensorMap* map, int t, int j, uint32_t bar_full) -> bool {
           if (static_cast<int>(kv_count) == p.test_drop_load) {   // test hook: this tile is never announced
             ++kv_count;
             return true;
@@ -264,9 +280,10 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           const uint32_t ph = (kv_count / C::kStages) & 1;
           if (!mbar_wait(bar_kv_empty(s), ph ^ 1, abort_flag, wait_ns, kTagKvEmpty)) return false;
           RSFA_TRACE_EV(0x200 + j);
-          mbar_arrive_expect_tx(bar_kv_full(s), C::kKvTileBytes);
+          if (bar_full == 0) bar_full = bar_kv_full(s);
+          mbar_arrive_expect_tx(bar_full, C::kKvTileBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
-            tma_load_4d(sKV + s * C::kKvTileBytes + bx * C::kKvBoxBytes, map, bar_kv_full(s), bx * 64,
+            tma_load_4d(sKV + s * C::kKvTileBytes + bx * C::kKvBoxBytes, map, bar_full, bx * 64,
                         key_tile(t, j) * kTileN, th[t], tb[t]);
           ++kv_count;
           return true;
@@ -275,26 +292,33 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           // K_0 first: its ring slot frees up while the previous item drains.  Then the Q tiles, which
           // wait for that item's last QK^T, and only then V_0, whose slot frees up last of all: behind
           // V_0 the Q loads, which come from DRAM, started 2000 clk later than they could.
-          if (nmax > 0) ok = load_kv(&maps.k, 0, 0);
+          ok = load_kv(&maps.k, 0, 0, bar_k_first(item_count));
           if (ok) ok = load_q(0);
           if (ok) ok = load_q(1);
-          if (ok && nmax > 0) ok = load_kv(&maps.v, 0, 0);
-          for (int j = 1; ok && j < nmax; ++j) {
-            ok = load_kv(&maps.k, 0, j);
-            if (ok) ok = load_kv(&maps.v, 0, j);
+          for (int j = 0; ok && j < nmax; ++j) {
+            // A barrier's turn comes again two steps later; by then its phase is over, because the ring slot that
+            // this load waits for is given back behind the MMAs of that step.
+            const bool tile0 = j < n[0];
+            ok = load_kv(&maps.v, 0, j, tile0 ? bar_p_full(0, 0, p0_steps) : bar_v_lone);
+            if (!ok) break;
+            if (j + 1 < nmax)   // n[1] <= n[0] + 1: a step that needs K_{j+1} is a step of tile 0
+              ok = load_kv(&maps.k, 0, j + 1, bar_p_full(0, 1, p0_steps));
+            else if (tile0)
+              mbar_arrive(bar_p_full(0, 1, p0_steps));   // no K_{j+1}
+            if (tile0) ++p0_steps;
           }
         } else {
           // Every Q tile has K/V tiles of its own, in the ring in the order in which the MMA warp uses them:
           // K^0_0 K^1_0, then per step V^0_j K^0_{j+1} V^1_j K^1_{j+1}.  A Q tile without work still gets its
           // Q (rows of a head past the last one read as zeros), so that its barriers keep step.
           for (int t = 0; ok && t < kNT; ++t) {
-            if (n[t] > 0) ok = load_kv(&maps.k, t, 0);
+            if (n[t] > 0) ok = load_kv(&maps.k, t, 0, 0u);
             if (ok && t < C::kQBufs) ok = load_q(t);
           }
           for (int j = 0; ok && j < nmax; ++j) {
             for (int t = 0; ok && t < kNT; ++t) {
-              if (j < n[t]) ok = load_kv(&maps.v, t, j);
-              if (ok && j + 1 < n[t]) ok = load_kv(&maps.k, t, j + 1);
+              if (j < n[t]) ok = load_kv(&maps.v, t, j, 0u);
+              if (ok && j + 1 < n[t]) ok = load_kv(&maps.k, t, j + 1, 0u);
             }
           }
         }
@@ -318,6 +342,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       const uint64_t desc_v0 = make_smem_desc_sw128(sKV, C::kKvBoxBytes, 1024);
       uint32_t kv_count = 0, item_count = 0;
       uint32_t p_count[kNT] = {0, 0};
+      uint32_t lone_count = 0;   // kPair: steps so far that only tile 1 had
       bool ok = true;
       while (ok) {
         const int slot = item_count & 1;
@@ -410,11 +435,11 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
               if (j >= n[t]) continue;
               ok = next_kv();   // V
               if (!ok) break;
-              ok = wait_all(bar_p_full(t, 0), p_count[t] & 1, kTagPFull);
+              ok = wait_all(bar_p_full(t, 0, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
               if (!ok) break;
               tc_fence_after_sync();
               issue_pv(t, kv_count % C::kStages, j > 0, 0, kTileN / 32, bar_pv0_done(t));
-              ok = wait_all(bar_p_full(t, 1), p_count[t] & 1, kTagPFull);
+              ok = wait_all(bar_p_full(t, 1, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
               if (!ok) break;
               ++p_count[t];
               tc_fence_after_sync();
@@ -433,9 +458,9 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           ++item_count;
           continue;
         }
-        const uint32_t base = kv_count;  // K_j at base + 2j, V_j at base + 2j + 1
+        const uint32_t base = kv_count;  // ring slots: K_j at base + 2j, V_j at base + 2j + 1
         if (nmax > 0) {
-          ok = wait_kv(base);
+          ok = wait_all(bar_k_first(item_count), (item_count >> 1) & 1, kTagKvFull);
           if (!ok) break;
           RSFA_TRACE_EV(0xa200);   // K_0 present
           for (int t = 0; ok && t < kNT; ++t) {
@@ -456,7 +481,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           umma_commit_elect(bar_kv_empty(base % C::kStages));
         }
         // Steady state, kept free of everything the end of an item needs: while both tiles have key tiles
-        // left after step j, every step is V_j, then per tile PV(j) in two halves and QK^T(j+1).  The MMA
+        // left after step j, every step is PV(j) in two halves and QK^T(j+1) per tile.  The MMA
         // warp is the pacemaker of the CTA: an extra test or call in this loop shows up in every step.
         const int n_lean = min(n[0], n[1]) - 1;
         int j0 = 0;
@@ -464,30 +489,21 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           const uint32_t vidx = base + 2 * j0 + 1;
           const uint32_t kidx = base + 2 * j0 + 2;
           const uint32_t vslot = vidx % C::kStages, kslot = kidx % C::kStages;
-          ok = wait_kv(vidx);
-          if (!ok) break;
-          RSFA_TRACE_EV(0x6000 + j0);                  // V_j present
 #pragma unroll
           for (int t = 0; t < kNT; ++t) {
-            ok = wait_all(bar_p_full(t, 0), p_count[t] & 1, kTagPFull);
+            ok = wait_all(bar_p_full(t, 0, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
             if (!ok) break;
             tc_fence_after_sync();
             RSFA_TRACE_EV(0x1000 + (t << 8) + j0);   // P half 0 seen
             issue_pv(t, vslot, j0 > 0, 0, kTileN / 32, bar_pv0_done(t));
             RSFA_TRACE_EV(0x2000 + (t << 8) + j0);   // PV half 0 issued
-            ok = wait_all(bar_p_full(t, 1), p_count[t] & 1, kTagPFull);
+            ok = wait_all(bar_p_full(t, 1, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
             if (!ok) break;
             ++p_count[t];
             tc_fence_after_sync();
             RSFA_TRACE_EV(0x3000 + (t << 8) + j0);   // P half 1 seen
             issue_pv(t, vslot, true, kTileN / 32, kTileN / 16, 0u);
             RSFA_TRACE_EV(0x4000 + (t << 8) + j0);   // PV half 1 issued
-            if (t == 0) {
-              ok = wait_kv(kidx);
-              if (!ok) break;
-              tc_fence_after_sync();
-            }
-            RSFA_TRACE_EV(0x9000 + (t << 8) + j0);   // K ready
             // behind the last MMAs of the step that read V_j and K_{j+1} the release of both slots rides along
             issue_qk(t, kslot, bar_s_full(t), j0 + 2 == n[t] ? bar_q_empty(t) : 0u,
                      t == kNT - 1 ? bar_kv_empty(vslot) : 0u, t == kNT - 1 ? bar_kv_empty(kslot) : 0u);
@@ -501,19 +517,21 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         for (int j = j0; ok && j < nmax; ++j) {
           const uint32_t vidx = base + 2 * j + 1;
           const uint32_t kidx = base + 2 * j + 2;
-          ok = wait_kv(vidx);
-          if (!ok) break;
-          RSFA_TRACE_EV(0x6000 + j);                  // V_j present
-          bool k_ready = false, folded = false;
+          if (j >= n[0]) {   // tile 1 alone
+            ok = wait_all(bar_v_lone, lone_count & 1, kTagKvFull);
+            if (!ok) break;
+            ++lone_count;
+          }
+          bool folded = false;
           for (int t = 0; ok && t < kNT; ++t) {
             if (j < n[t]) {
-              ok = wait_all(bar_p_full(t, 0), p_count[t] & 1, kTagPFull);
+              ok = wait_all(bar_p_full(t, 0, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
               if (!ok) break;
               tc_fence_after_sync();
               RSFA_TRACE_EV(0x1000 + (t << 8) + j);   // P half 0 seen
               issue_pv(t, vidx % C::kStages, j > 0, 0, kTileN / 32, bar_pv0_done(t));
               RSFA_TRACE_EV(0x2000 + (t << 8) + j);   // PV half 0 issued
-              ok = wait_all(bar_p_full(t, 1), p_count[t] & 1, kTagPFull);
+              ok = wait_all(bar_p_full(t, 1, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
               if (!ok) break;
               ++p_count[t];
               tc_fence_after_sync();
@@ -522,13 +540,6 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
               RSFA_TRACE_EV(0x4000 + (t << 8) + j);   // PV half 1 issued
             }
             if (j + 1 < n[t]) {
-              if (!k_ready) {
-                ok = wait_kv(kidx);
-                if (!ok) break;
-                tc_fence_after_sync();
-                k_ready = true;
-              }
-              RSFA_TRACE_EV(0x9000 + (t << 8) + j);   // K ready
               folded = (t == kNT - 1);   // the last MMAs of the step: the release of both slots rides along
               issue_qk(t, kidx % C::kStages, bar_s_full(t), j + 2 == n[t] ? bar_q_empty(t) : 0u,
                        folded ? bar_kv_empty(vidx % C::kStages) : 0u, folded ? bar_kv_empty(kidx % C::kStages) : 0u);
@@ -536,10 +547,6 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
             }
           }
           if (!ok) break;
-          if (j + 1 < nmax && !k_ready) {  // tile loaded for a Q tile that did not need it: still consume it
-            ok = wait_kv(kidx);
-            if (!ok) break;
-          }
           if (!folded)
             umma_commit2_elect(bar_kv_empty(vidx % C::kStages), j + 1 < nmax ? bar_kv_empty(kidx % C::kStages) : 0u);
           RSFA_TRACE_EV(0x7000 + j);   // iteration end
@@ -702,7 +709,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           tmem_st_x32(tS, pk);
           tmem_wait_st();
           tc_fence_before_sync();
-          mbar_arrive(bar_p_full(t, 0));
+          mbar_arrive(bar_p_full(t, 0, s_count - 1));
           RSFA_TRACE_EV(0x4000 + j);   // half 0 handed over
         }
         {
@@ -717,7 +724,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           tmem_st_x32(tS + 32, pk);
           tmem_wait_st();
           tc_fence_before_sync();
-          mbar_arrive(bar_p_full(t, 1));
+          mbar_arrive(bar_p_full(t, 1, s_count - 1));
         }
         RSFA_TRACE_EV(0x5000 + j);   // half 1 handed over
       }
@@ -744,7 +751,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           unpack_f32x2(r, m_used, l);
           tmem_wait_st();
           tc_fence_before_sync();
-          mbar_arrive(bar_p_full(t, half));
+          mbar_arrive(bar_p_full(t, half, s_count - 1));
         }
         if (!ok) break;
         ++j;

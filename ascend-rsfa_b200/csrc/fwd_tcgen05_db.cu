@@ -47,6 +47,14 @@ struct DbCfg {
   // One Q tile at D <= 64 needs half of everything (192 tensor-memory columns, 97 KB): two CTAs per SM.
   static constexpr int kCtasPerSm = (NT == 1 && D != 256) ? 2 : 1;
   static constexpr int kTmemCols = 512 / kCtasPerSm;
+  // One Q tile: the bytes of the ring entry that a step needs, (V_j, K_{j+2}), are counted on the barrier on which
+  // the softmax hands over P_j, so the MMA warp waits once per step.  The loads run up to kStages entries ahead of
+  // the softmax: kTurns such barriers are used in turn (kTurns >= kStages: a barrier's turn comes again when the
+  // ring slot of the step that had it is given back).  D = 256: S = 1024 causal 321 -> 308 us, S = 2048 causal 542 ->
+  // 512; D = 64 1 %.  (One MMA warp for a pair of tiles, which could have the same, is 5 % slower: 24 MMAs and
+  // their commits per step are more than one warp can issue.)
+  static constexpr bool kJoint = (NT == 1);
+  static constexpr int kTurns = kJoint ? 4 : 0;
   static constexpr int kStages = (D == 256) ? 3 : (kCtasPerSm == 2 ? 4 : (D == 128 ? 4 : 6));
   // D = 256 has a warpgroup of its own for the epilogue (warps 8-11; a warp reads the tensor-memory
   // lanes 32 * (warp % 4) ...): the single softmax group goes straight on to the next work item and
@@ -66,7 +74,7 @@ struct DbCfg {
   static constexpr int kStageBufs = (D == 256) ? 2 : 1;
   static constexpr int kStageBytes = kStageBufs * kRowsDb * 128;
 
-  static constexpr int kNumBarriers = 4 * NT + 4 * NT + NT + 2 * kStages + 4 + 2;
+  static constexpr int kNumBarriers = 4 * NT + 4 * NT + NT + 2 * kStages + 4 + 2 + kTurns;
   // D = 256 leaves 128 tensor-memory columns free: Q lives there as the A operand of QK^T.  Those
   // MMAs then read only K from shared memory (with both operands there, N = 64 took 65 clk instead
   // of 32 and the MMA warp was the limit), and Q needs no shared-memory buffer of its own: it comes
@@ -103,7 +111,10 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
   auto bar_pv_done = [&](int t) { return sBar + 8u * (2 * NT + t); };   // one completion per key tile
   auto bar_o_full = [&](int t) { return sBar + 8u * (3 * NT + t); };    // one completion per work item
   auto bar_s_full = [&](int t, int b) { return sBar + 8u * (4 * NT + 2 * t + b); };
-  auto bar_p_full = [&](int t, int b) { return sBar + 8u * (6 * NT + 2 * t + b); };
+  // P of key tile `step` (counted over all work items) of Q tile t, in buffer b
+  auto bar_p_full = [&](int t, int b, uint32_t step) {
+    return C::kJoint ? sBar + 8u * (C::kNumBarriers - C::kTurns + (step & 3u)) : sBar + 8u * (6 * NT + 2 * t + b);
+  };
   auto bar_kv_full = [&](int s) { return sBar + 8u * (8 * NT + s); };
   auto bar_kv_empty = [&](int s) { return sBar + 8u * (8 * NT + C::kStages + s); };
   const uint32_t bar_sched_full0 = sBar + 8u * (9 * NT + 2 * C::kStages);  // 2 slots
@@ -132,9 +143,10 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       mbar_init(bar_o_full(t), 1);
       for (int b = 0; b < 2; ++b) {
         mbar_init(bar_s_full(t, b), 1);
-        mbar_init(bar_p_full(t, b), kRowsDb);
+        if (!C::kJoint) mbar_init(bar_p_full(t, b, 0), kRowsDb);
       }
     }
+    for (uint32_t i = 0; i < static_cast<uint32_t>(C::kTurns); ++i) mbar_init(bar_p_full(0, 0, i), kRowsDb + 1);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_kv_full(s), 1);
       mbar_init(bar_kv_empty(s), NT);   // one commit per MMA warp
@@ -171,7 +183,8 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
     // ================================================================ producer
     if (lane == 0) {
       RSFA_TRACE_DECL(3);
-      uint32_t kv_count = 0;
+      uint32_t kv_count = 0;       // ring entries so far
+      uint32_t first_count = 0, step_count = 0;   // kJoint: of those, the ones in front of an item's steps / its steps
       uint32_t claim_count = 0;    // work items claimed / published so far
       uint32_t publish_count = 0;
       bool ok = true;
@@ -226,17 +239,17 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
           claimed = true;
         }
         // one ring entry: tile A (K_0 or V_j) and, when it exists, tile B (K_1 or K_{j+2})
-        auto load_pair = [&](const CUtensorMap* map_a, int ja, bool has_b, int jb) -> bool {
+        auto load_pair = [&](const CUtensorMap* map_a, int ja, bool has_b, int jb, uint32_t bar_full) -> bool {
           const uint32_t s = kv_count % C::kStages;
           const uint32_t ph = (kv_count / C::kStages) & 1;
           if (!mbar_wait(bar_kv_empty(s), ph ^ 1, abort_flag, wait_ns, kTagKvEmpty)) return false;
           RSFA_TRACE_EV(0x200 + ja);
-          mbar_arrive_expect_tx(bar_kv_full(s), has_b ? C::kSlotBytes : C::kKvBytes);
+          mbar_arrive_expect_tx(bar_full, has_b ? C::kSlotBytes : C::kKvBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
-            tma_load_4d(sKV + s * C::kSlotBytes + bx * C::kKvBoxBytes, map_a, bar_kv_full(s), bx * 64, ja * kKeysDb, h, b);
+            tma_load_4d(sKV + s * C::kSlotBytes + bx * C::kKvBoxBytes, map_a, bar_full, bx * 64, ja * kKeysDb, h, b);
           if (has_b) {
             for (int bx = 0; bx < C::kBoxes; ++bx)
-              tma_load_4d(sKV + s * C::kSlotBytes + C::kKvBytes + bx * C::kKvBoxBytes, &maps.k, bar_kv_full(s), bx * 64,
+              tma_load_4d(sKV + s * C::kSlotBytes + C::kKvBytes + bx * C::kKvBoxBytes, &maps.k, bar_full, bx * 64,
                           jb * kKeysDb, h, b);
           }
           ++kv_count;
@@ -249,19 +262,21 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
           ok = mbar_wait(bar_kv_empty(s), ph ^ 1, abort_flag, wait_ns, kTagKvEmpty);
           if (!ok) break;
           RSFA_TRACE_EV(0x100);
-          mbar_arrive_expect_tx(bar_kv_full(s), C::kQTileBytes);
+          const uint32_t bar = bar_kv_full(first_count++ % C::kStages);
+          mbar_arrive_expect_tx(bar, C::kQTileBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
-            tma_load_4d(sKV + s * C::kSlotBytes + bx * C::kQBoxBytes, &maps.q, bar_kv_full(s), bx * 64, row0, h, b);
+            tma_load_4d(sKV + s * C::kSlotBytes + bx * C::kQBoxBytes, &maps.q, bar, bx * 64, row0, h, b);
           ++kv_count;
         }
-        ok = load_pair(&maps.k, 0, nmax > 1, 1);
+        ok = load_pair(&maps.k, 0, nmax > 1, 1, bar_kv_full((C::kJoint ? first_count++ : kv_count) % C::kStages));
         for (int j = 0; ok && j < nmax; ++j) {
           if (j == j_next) {
             if (!claimed) next = claim();
             ok = publish(next);
             if (!ok) break;
           }
-          ok = load_pair(&maps.v, j, j + 2 < nmax, j + 2);
+          ok = load_pair(&maps.v, j, j + 2 < nmax, j + 2,
+                         C::kJoint ? bar_p_full(0, 0, step_count++) : bar_kv_full(kv_count % C::kStages));
         }
       }
     }
@@ -309,6 +324,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
     const uint64_t desc_v0 = make_smem_desc_sw128(sKV, C::kKvBoxBytes, 1024);
     const uint32_t col_o = tmem_u + C::col_o(t);
     uint32_t kv_count = 0, item_count = 0;
+    uint32_t first_count = 0, step_count = 0;   // kJoint: as in the producer
     uint32_t p_count[2] = {0, 0};
     bool ok = true;
     while (ok) {
@@ -365,8 +381,9 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         // slabs an SS-form MMA would read); the copies run in order behind the last item's MMAs and in
         // front of the QK^T issued below, and the slot is free again when they are complete.
         const uint32_t qs = kv_count % C::kStages;
-        ok = wait_all(bar_kv_full(qs), (kv_count / C::kStages) & 1, kTagQFull);
+        ok = wait_all(bar_kv_full(first_count % C::kStages), (first_count / C::kStages) & 1, kTagQFull);
         if (!ok) break;
+        ++first_count;
         tc_fence_after_sync();
         RSFA_TRACE_EV(0x4000);   // Q present
         const uint64_t qd = desc_k0 + static_cast<uint64_t>((qs * C::kSlotBytes) >> 4);
@@ -385,8 +402,10 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       // entry 0: (K_0, K_1) -> S_t[0], S_t[1]
       {
         const uint32_t s = kv_count % C::kStages;
-        ok = wait_all(bar_kv_full(s), (kv_count / C::kStages) & 1, kTagKvFull);
+        const uint32_t entry = C::kJoint ? first_count : kv_count;
+        ok = wait_all(bar_kv_full(entry % C::kStages), (entry / C::kStages) & 1, kTagKvFull);
         if (!ok) break;
+        ++first_count;
         tc_fence_after_sync();
         RSFA_TRACE_EV(0x60ff);   // (K_0, K_1) present
         for (int j = 0; j < 2; ++j) {
@@ -401,13 +420,20 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       for (int j = 0; ok && j < nmax; ++j) {
         const int buf = j & 1;
         const uint32_t s = kv_count % C::kStages;
-        ok = wait_all(bar_kv_full(s), (kv_count / C::kStages) & 1, kTagKvFull);
-        if (!ok) break;
-        RSFA_TRACE_EV(0x6000 + j);   // entry present
-        if (j < n) {
-          ok = wait_all(bar_p_full(t, buf), p_count[buf] & 1, kTagPFull);
+        if constexpr (!C::kJoint) {
+          ok = wait_all(bar_kv_full(s), (kv_count / C::kStages) & 1, kTagKvFull);
           if (!ok) break;
-          ++p_count[buf];
+          RSFA_TRACE_EV(0x6000 + j);   // entry present
+        }
+        if (C::kJoint || j < n) {
+          if constexpr (C::kJoint) {
+            ok = wait_all(bar_p_full(t, buf, step_count), (step_count >> 2) & 1, kTagPFull);
+            ++step_count;
+          } else {
+            ok = wait_all(bar_p_full(t, buf, 0), p_count[buf] & 1, kTagPFull);
+            ++p_count[buf];
+          }
+          if (!ok) break;
           tc_fence_after_sync();
           RSFA_TRACE_EV(0x1000 + j);   // P seen
           if (C::kEpi && j == 0 && item_count > 0) {
@@ -547,7 +573,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
           tmem_st_x32(tS, pk);
           tmem_wait_st();
           tc_fence_before_sync();
-          mbar_arrive(bar_p_full(t, buf));
+          mbar_arrive(bar_p_full(t, buf, pv_count + j));
           RSFA_TRACE_EV(0x5000 + j);   // P handed over
         }
         if (!ok) break;
@@ -570,7 +596,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
           unpack_f32x2(r, m_used, l);
           tmem_wait_st();
           tc_fence_before_sync();
-          mbar_arrive(bar_p_full(t, buf));
+          mbar_arrive(bar_p_full(t, buf, pv_count + j));
           ++j;
         }
       }
