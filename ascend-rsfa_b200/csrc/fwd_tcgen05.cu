@@ -82,7 +82,7 @@ struct Cfg {
   static constexpr int kQBoxBytes = kTileM * 128;             // 128 rows x 128 B
   static constexpr int kKvBoxBytes = kTileN * 128;
   static constexpr int kStageBytes = kTileM * 128;            // epilogue staging: 128 rows x 64 columns
-  static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4 + 2 + 2;
+  static constexpr int kNumBarriers = 2 * kNT + 2 * kStages + 6 * kNT + 4 + 2 + 2 * kNT;
   static constexpr int kMlBytes = (kMode == kSplitKeys) ? kNT * kTileM * 8 : 0;   // (m, l) of every row, twice
   static constexpr int kSmemBytes = kQBufs * kQTileBytes + kStages * kKvTileBytes + kNT * kStageBytes + 1024 /*align*/ +
                                     kNumBarriers * 8 + 80 + kMlBytes;
@@ -114,20 +114,22 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   auto bar_kv_full = [&](int s) { return sBar + 8u * (2 * kNT + s); };
   auto bar_kv_empty = [&](int s) { return sBar + 8u * (2 * kNT + C::kStages + s); };
   auto bar_s_full = [&](int t) { return sBar + 8u * (2 * kNT + 2 * C::kStages + t); };
-  // P_t is handed to the MMA warp in two halves of 64 keys so the first PV MMAs start early.  kPair: the MMA
-  // warp needs V_j with the first half of P_0(j) and K_{j+1} with the second, so the bytes of those loads are
-  // counted on the same barriers and one wait says both.  The loads run up to two steps ahead of the softmax:
-  // tile 0's barriers are two pairs used in turn (`step` = its key tiles so far).  Two waits per step less (four
-  // instead of six for the warp that paces the CTA): (16, 16, 4096, 128) causal 911 -> 894 us, (128, 8, 2048, 128)
-  // 1925 -> 1877, S = 1024 causal 86.6 -> 84.7.
-  const uint32_t bar_p0_odd = sBar + 8u * (C::kNumBarriers - 2);
+  // P_t is handed to the MMA warp in two halves of 64 keys so the first PV MMAs start early.  The MMA warp needs
+  // V_j with the first half of P(j) and K_{j+1} with the second, so the bytes of those loads are counted on the
+  // same barriers and one wait says both; with K/V tiles shared by the Q tiles (kPair) on those of tile 0.  The
+  // loads run up to two steps ahead of the softmax: such barriers are two pairs used in turn (`step` = the key
+  // tiles of that Q tile so far).  Two waits per step less (four instead of six for the warp that paces the CTA):
+  // (16, 16, 4096, 128) causal 911 -> 894 us, (128, 8, 2048, 128) 1925 -> 1877, S = 1024 causal 86.6 -> 84.7, 8 heads
+  // of S = 2048 (kSplitKeys) 22.4 -> 21.6.
+  auto joint = [](int t) { return kMode != kPair || t == 0; };
   auto bar_p_full = [&](int t, int half, uint32_t step) {
-    const uint32_t even = sBar + 8u * (3 * kNT + 2 * C::kStages + 2 * t + half);
-    return (kMode == kPair && t == 0 && (step & 1) != 0) ? bar_p0_odd + 8u * half : even;
+    return (joint(t) && (step & 1) != 0) ? sBar + 8u * (C::kNumBarriers - 2 * kNT + 2 * t + half)
+                                         : sBar + 8u * (3 * kNT + 2 * C::kStages + 2 * t + half);
   };
-  auto p_parity = [](int t, uint32_t step) -> uint32_t { return (kMode == kPair && t == 0) ? (step >> 1) & 1 : step & 1; };
-  // kPair: what is not counted on those: K_0 of an item (two in turn), V_j of a step that only tile 1 has
-  auto bar_k_first = [&](uint32_t item_count) { return bar_kv_full(item_count & 1); };
+  auto p_parity = [&](int t, uint32_t step) -> uint32_t { return joint(t) ? (step >> 1) & 1 : step & 1; };
+  // what is not counted on those: K_0 of an item (of tile t; the items in which it has work, counted by `first`, take
+  // two barriers in turn), V_j of a step that only tile 1 of a pair has
+  auto bar_k_first = [&](int t, uint32_t first) { return bar_kv_full(2 * t + (first & 1)); };
   const uint32_t bar_v_lone = bar_kv_full(2);
   auto bar_o_full = [&](int t) { return sBar + 8u * (5 * kNT + 2 * C::kStages + t); };
   // completion of the PV MMAs of a tile's first 64 keys (waited on only by the softmax slow path)
@@ -158,9 +160,9 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       mbar_init(bar_q_full(t), 1);
       mbar_init(bar_q_empty(t), 1);
       mbar_init(bar_s_full(t), 1);
-      for (uint32_t step = 0; step < (kMode == kPair && t == 0 ? 2u : 1u); ++step) {
-        mbar_init(bar_p_full(t, 0, step), kTileM + (kMode == kPair && t == 0 ? 1 : 0));
-        mbar_init(bar_p_full(t, 1, step), kTileM + (kMode == kPair && t == 0 ? 1 : 0));
+      for (uint32_t step = 0; step < (joint(t) ? 2u : 1u); ++step) {
+        mbar_init(bar_p_full(t, 0, step), kTileM + (joint(t) ? 1 : 0));
+        mbar_init(bar_p_full(t, 1, step), kTileM + (joint(t) ? 1 : 0));
       }
       mbar_init(bar_o_full(t), 1);
       mbar_init(bar_pv0_done(t), 1);
@@ -219,7 +221,8 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       RSFA_TRACE_DECL(3);
       uint32_t kv_count = 0;   // K/V tiles loaded so far (ring position)
       uint32_t item_count = 0; // work items started so far
-      uint32_t p0_steps = 0;   // kPair: key tiles of tile 0 so far
+      uint32_t steps[kNT] = {0, 0};   // key tiles of each Q tile so far
+      uint32_t first[kNT] = {0, 0};   // items in which it had work (not kPair)
       bool ok = true;
       while (ok) {
         // fetch the next work item and publish it to the other roles
@@ -280,7 +283,6 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           const uint32_t ph = (kv_count / C::kStages) & 1;
           if (!mbar_wait(bar_kv_empty(s), ph ^ 1, abort_flag, wait_ns, kTagKvEmpty)) return false;
           RSFA_TRACE_EV(0x200 + j);
-          if (bar_full == 0) bar_full = bar_kv_full(s);
           mbar_arrive_expect_tx(bar_full, C::kKvTileBytes);
           for (int bx = 0; bx < C::kBoxes; ++bx)
             tma_load_4d(sKV + s * C::kKvTileBytes + bx * C::kKvBoxBytes, map, bar_full, bx * 64,
@@ -292,33 +294,39 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           // K_0 first: its ring slot frees up while the previous item drains.  Then the Q tiles, which
           // wait for that item's last QK^T, and only then V_0, whose slot frees up last of all: behind
           // V_0 the Q loads, which come from DRAM, started 2000 clk later than they could.
-          ok = load_kv(&maps.k, 0, 0, bar_k_first(item_count));
+          ok = load_kv(&maps.k, 0, 0, bar_k_first(0, item_count));
           if (ok) ok = load_q(0);
           if (ok) ok = load_q(1);
           for (int j = 0; ok && j < nmax; ++j) {
             // A barrier's turn comes again two steps later; by then its phase is over, because the ring slot that
             // this load waits for is given back behind the MMAs of that step.
             const bool tile0 = j < n[0];
-            ok = load_kv(&maps.v, 0, j, tile0 ? bar_p_full(0, 0, p0_steps) : bar_v_lone);
+            ok = load_kv(&maps.v, 0, j, tile0 ? bar_p_full(0, 0, steps[0]) : bar_v_lone);
             if (!ok) break;
             if (j + 1 < nmax)   // n[1] <= n[0] + 1: a step that needs K_{j+1} is a step of tile 0
-              ok = load_kv(&maps.k, 0, j + 1, bar_p_full(0, 1, p0_steps));
+              ok = load_kv(&maps.k, 0, j + 1, bar_p_full(0, 1, steps[0]));
             else if (tile0)
-              mbar_arrive(bar_p_full(0, 1, p0_steps));   // no K_{j+1}
-            if (tile0) ++p0_steps;
+              mbar_arrive(bar_p_full(0, 1, steps[0]));   // no K_{j+1}
+            if (tile0) ++steps[0];
           }
         } else {
           // Every Q tile has K/V tiles of its own, in the ring in the order in which the MMA warp uses them:
           // K^0_0 K^1_0, then per step V^0_j K^0_{j+1} V^1_j K^1_{j+1}.  A Q tile without work still gets its
           // Q (rows of a head past the last one read as zeros), so that its barriers keep step.
           for (int t = 0; ok && t < kNT; ++t) {
-            if (n[t] > 0) ok = load_kv(&maps.k, t, 0, 0u);
+            if (n[t] > 0) ok = load_kv(&maps.k, t, 0, bar_k_first(t, first[t]++));
             if (ok && t < C::kQBufs) ok = load_q(t);
           }
           for (int j = 0; ok && j < nmax; ++j) {
             for (int t = 0; ok && t < kNT; ++t) {
-              if (j < n[t]) ok = load_kv(&maps.v, t, j, 0u);
-              if (ok && j + 1 < n[t]) ok = load_kv(&maps.k, t, j + 1, 0u);
+              if (j >= n[t]) continue;
+              ok = load_kv(&maps.v, t, j, bar_p_full(t, 0, steps[t]));
+              if (!ok) break;
+              if (j + 1 < n[t])
+                ok = load_kv(&maps.k, t, j + 1, bar_p_full(t, 1, steps[t]));
+              else
+                mbar_arrive(bar_p_full(t, 1, steps[t]));   // no K of a next step
+              ++steps[t];
             }
           }
         }
@@ -343,6 +351,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
       uint32_t kv_count = 0, item_count = 0;
       uint32_t p_count[kNT] = {0, 0};
       uint32_t lone_count = 0;   // kPair: steps so far that only tile 1 had
+      uint32_t first[kNT] = {0, 0};   // as in the producer
       bool ok = true;
       while (ok) {
         const int slot = item_count & 1;
@@ -397,19 +406,9 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           }
           __syncwarp();
         };
-        auto wait_kv = [&](uint32_t idx) -> bool {
-          return wait_all(bar_kv_full(idx % C::kStages), (idx / C::kStages) & 1, kTagKvFull);
-        };
-
         if constexpr (kMode != kPair) {
           // K/V tiles of their own for each Q tile: a ring entry is read by one batch of MMAs and given back
-          // behind it.
-          auto next_kv = [&]() -> bool {
-            if (!wait_kv(kv_count)) return false;
-            tc_fence_after_sync();
-            return true;
-          };
-          // Q buffer to give back behind QK^T of step j of tile t (0: none): its own one behind its last step,
+          // behind it.  Q buffer to give back behind QK^T of step j of tile t (0: none): its own one behind its last step,
           // the shared one behind the last QK^T of the item.
           auto q_release = [&](int t, int j) -> uint32_t {
             if (j + 1 != n[t]) return 0u;
@@ -418,7 +417,8 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           };
           for (int t = 0; ok && t < kNT; ++t) {
             if (n[t] > 0) {
-              ok = next_kv();
+              ok = wait_all(bar_k_first(t, first[t]), (first[t] >> 1) & 1, kTagKvFull);
+              ++first[t];
               if (ok && t < C::kQBufs) ok = wait_all(bar_q_full(t), item_count & 1, kTagQFull);
               if (!ok) break;
               tc_fence_after_sync();
@@ -433,8 +433,6 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
           for (int j = 0; ok && j < nmax; ++j) {
             for (int t = 0; ok && t < kNT; ++t) {
               if (j >= n[t]) continue;
-              ok = next_kv();   // V
-              if (!ok) break;
               ok = wait_all(bar_p_full(t, 0, p_count[t]), p_parity(t, p_count[t]), kTagPFull);
               if (!ok) break;
               tc_fence_after_sync();
@@ -447,8 +445,6 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
               umma_commit_elect(bar_kv_empty(kv_count % C::kStages));
               ++kv_count;
               if (j + 1 < n[t]) {
-                ok = next_kv();   // K of the next step
-                if (!ok) break;
                 issue_qk(t, kv_count % C::kStages, bar_s_full(t), q_release(t, j + 1), bar_kv_empty(kv_count % C::kStages));
                 ++kv_count;
               }
@@ -460,7 +456,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
         }
         const uint32_t base = kv_count;  // ring slots: K_j at base + 2j, V_j at base + 2j + 1
         if (nmax > 0) {
-          ok = wait_all(bar_k_first(item_count), (item_count >> 1) & 1, kTagKvFull);
+          ok = wait_all(bar_k_first(0, item_count), (item_count >> 1) & 1, kTagKvFull);
           if (!ok) break;
           RSFA_TRACE_EV(0xa200);   // K_0 present
           for (int t = 0; ok && t < kNT; ++t) {
