@@ -70,6 +70,8 @@ def main():
             for bm, bn in CANDIDATES:
                 ms = 0.0
                 good = True
+                # the pair kernel of the tile itself: a request alone leaves the choice of its forms to the library
+                fa.set_option("tcgen05_variant", 1 if bn == 64 else (2 if D == 64 else 0))
                 for scale in scales:
                     path, tm, tn = fa.select_path(S, D, causal, scale, bm, bn)
                     assert (path, tm, tn) == (1, bm, bn), "tile (%d,%d) is not instantiated" % (bm, bn)
@@ -80,6 +82,7 @@ def main():
                         good = False
                         break
                     ms += time_tile(q, k, v, causal, scale, bm, bn, args.iters)
+                fa.set_option("tcgen05_variant", -1)
                 if not good:
                     print("S=%d D=%d causal=%d tile (%d,%d): WRONG, not timed" % (S, D, causal, bm, bn))
                     continue
