@@ -57,10 +57,12 @@ def measure(fa, dev, hbm_gbs, shape, causal=False, sm_scale=0.5, iters=400, chec
     torch.cuda.synchronize()
     us = ev0.elapsed_time(ev1) / iters * 1e3
     tc = fa.select_path(S, D, causal, sm_scale, bm, bn)[0] == 1
+    one_tile = sm_scale > 0 and (S <= 128 if D <= 64 else S <= 64 and D == 128)   # csrc/fwd_short.cu
     rec = {"shape": [B, H, S, D], "causal": bool(causal), "us_per_call": us, "bytes_per_call": nbytes,
            "gb_per_s": nbytes / (us * 1e-6) / 1e9,
            "frac_of_measured_hbm": (nbytes / (us * 1e-6) / 1e9 / hbm_gbs) if hbm_gbs else None,
-           "kernel": "tcgen05 (one key tile per work item)" if tc else "short-sequence (mma.sync)",
+           "kernel": ("short (TMA ring, mma.sync)" if one_tile else
+                      "tcgen05 (one key tile per Q tile)" if tc else "general (mma.sync)"),
            "input_sets_rotated": sets}
     if check:
         from oracle.attention_ref import attention_fp32, error_metrics

@@ -137,9 +137,9 @@ RSFA_API int rsfa_get_tiling(int B, int H, int S, int D, int causal, int* block_
 /*
  * Which kernel family rsfa_fwd would use for this problem, and the tile it would run
  * (after snapping block_m/block_n).  Counterpart of the dispatch in _attention.forward (:564-610).
- * tile_m / tile_n may be NULL.  The tcgen05 kernels run every shape with sm_scale > 0 except head
- * dimension 16 at S <= 128 and sequences of at most 64 keys at D <= 64, which the short-sequence
- * kernel serves (measured per call; the batch size does not enter).
+ * tile_m / tile_n may be NULL.  The answer goes by size alone: the tcgen05 family for every shape with
+ * sm_scale > 0 except head dimension 16 at S <= 128 and sequences of at most 64 keys at D <= 64; which
+ * form of a kernel, or the kernel for a single key tile, then runs is left open (see RSFA_PATH_*).
  */
 RSFA_API int rsfa_select_path(int S, int D, int causal, float sm_scale, int block_m, int block_n, int dtype,
                      int* path, int* tile_m, int* tile_n);
@@ -178,9 +178,8 @@ RSFA_API long long rsfa_launch_count(void);
 
 /*
  * Tuning / test knobs.  Names: "force_path" (-1 auto, 0 generic, 1 tcgen05),
- * "wait_limit_ms" (bound of every in-kernel wait, default 2000), "tcgen05_variant" (-1: the requested tile if
- * instantiated, else the tile table, and at D = 64 with 128-key tiles the separate-P kernel followed
- * by a second launch over the work items it could not finish; 0 / 1 force the single-buffered 128-key /
+ * "wait_limit_ms" (bound of every in-kernel wait, default 2000), "tcgen05_variant" (-1: by size,
+ * see block_m / block_n of rsfa_fwd; 0 / 1 force the pair form of the single-buffered 128-key /
  * double-buffered 64-key kernel for D <= 128; 2 forces 128-key tiles with the separate-P kernel where
  * it exists), "host_slab_heads"
  * (heads per staging slab of rsfa_fwd_host, 0 = automatic), "pdl" (1, the default: the tcgen05 kernels
