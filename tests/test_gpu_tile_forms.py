@@ -106,3 +106,32 @@ def test_single_q_tiles_follow_a_growing_maximum(fa, cuda_device):
     v = torch.randn(1, 2, S, 64, generator=g).half()
     for causal in (False, True):
         agree(fa, cuda_device, q, k, v, causal, 1.0)
+
+
+@pytest.mark.parametrize("B,H,S,D", [(2, 3, 640, 128), (30, 8, 100, 128), (3, 5, 300, 64), (2, 3, 520, 32)])
+def test_storage_orders_agree_with_the_pair_kernel(fa, cuda_device, B, H, S, D):
+    g = torch.Generator(device=cuda_device).manual_seed(S)
+    rand = lambda *shape: torch.randn(shape, generator=g, device=cuda_device).half()  # noqa: E731
+    forms = {
+        "bshd": [rand(B, S, H, D).transpose(1, 2) for _ in range(3)],
+        "hbsd": [rand(H, B, S, D).transpose(0, 1) for _ in range(3)],
+        "packed qkv": list(rand(B, S, 3, H, D).permute(2, 0, 3, 1, 4).unbind(0)),
+        "padded rows": [rand(B, H, S, D + 8)[..., :D] for _ in range(3)],
+        "sliced heads": [rand(B, 2 * H, S + 3, D)[:, 1::2, 2:S + 2] for _ in range(3)],
+        "one batch, odd stride": [rand(3 * H * S * D + 24)[:H * S * D].view(1, H, S, D) for _ in range(3)],
+    }
+    u = 2.0 ** -11
+    for name, (q, k, v) in forms.items():
+        for causal in (False, True):
+            o = fa.attention(q, k, v, causal, 0.15, 128, 128)
+            fa.set_option("tcgen05_variant", 0)
+            try:
+                pair = fa.attention(q, k, v, causal, 0.15, 128, 128)
+            finally:
+                fa.set_option("tcgen05_variant", -1)
+            torch.cuda.synchronize()
+            fa.device_status()
+            assert o.stride() == pair.stride(), name
+            # each is within (2 u + S 2^-19) max|v| of the exact result (see agree)
+            limit = 2 * (2 * u + S * 2.0 ** -19) * float(v.float().abs().max())
+            assert float((o.float() - pair.float()).abs().max()) <= limit, (name, causal)
