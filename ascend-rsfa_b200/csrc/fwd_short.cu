@@ -23,10 +23,10 @@
 // Measured on 4096 heads (us per launch from a graph of launches, inputs rotated; before = the kernel that had
 // the size: fwd_generic at S <= 64, D <= 64 and D = 16, the tcgen05 kernels otherwise; floor = bytes at the
 // measured copy rate, 6.55 TB/s):
-//   S = 64 D = 64     72.3 -> 23.5 (floor 20.5)     S = 64 D = 128        95.5 -> 48.9 (floor 41.0)
-//   S = 100 D = 32    84.0 -> 42.1 (floor 16.0)     the same, causal      84.0 -> 31.6
+//   S = 64 D = 64     72.3 -> 23.0 (floor 20.5)     S = 64 D = 128        95.5 -> 48.5 (floor 41.0)
+//   S = 100 D = 32    84.0 -> 40.1 (floor 16.0)     the same, causal      84.0 -> 31.6
 //   S = 128 D = 64    72.5 -> 64.9 (floor 41.0)     the same, causal      84.8 -> 51
-//   S = 128 D = 16    57.3 -> 35   (floor 10.2)     S = 30 D = 64 (x 2)  109.9 -> 22.6 (floor 19.2)
+//   S = 128 D = 16    57.3 -> 29.5 (floor 10.2)     S = 30 D = 64 (x 2)  109.9 -> 22.6 (floor 19.2)
 // and at 2 to 64 heads, where latency is all there is: S = 128 D = 64 5.7 -> 4.1, S = 64 D = 128 6.8 -> 3.5.
 #include "../../include/rsfa.h"
 #include "tcgen05_common.cuh"
@@ -99,8 +99,9 @@ __device__ __forceinline__ uint32_t box_offset(int row, int chunk) {
   return static_cast<uint32_t>(row * kRowBytes + ((chunk ^ swizzle) << 4));
 }
 
-// kKeys: the key capacity of a warp's score registers (64 or 128), S <= kKeys.
-template <int D, int kKeys, bool kBf16>
+// kKeys: the key capacity of a warp's score registers (32, 64, 96 or 128), S <= kKeys.  kAll: no causal mask, and
+// kKeys is S rounded up to 32: every row sees every step of 32 keys.
+template <int D, int kKeys, bool kBf16, bool kAll>
 __global__ void __launch_bounds__(32 * kMaxWarpsShort, kCtasPerSmShort)
 fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, const ShortPlan plan) {
   constexpr int kSteps = kKeys / 32;               // steps of 32 keys
@@ -199,7 +200,7 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
     float s[kSteps][4][4];
 #pragma unroll
     for (int st = 0; st < kSteps; ++st) {
-      if (st == 0 || st < n_steps) {
+      if (kAll || st == 0 || st < n_steps) {
         // K fragments of up to four slices at a time: their loads go out together
 #pragma unroll
         for (int bx = 0; bx < kBoxes; ++bx) {
@@ -226,8 +227,8 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
     float m_lo = -INFINITY, m_hi = -INFINITY;
 #pragma unroll
     for (int st = 0; st < kSteps; ++st) {
-      if (st == 0 || st < n_steps) {
-        if (st * 32 + 31 > lim_all) {
+      if (kAll || st == 0 || st < n_steps) {
+        if ((!kAll || st == kSteps - 1) && st * 32 + 31 > lim_all) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
 #pragma unroll
@@ -257,7 +258,7 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
     float acc[D / 8][4];
 #pragma unroll
     for (int st = 0; st < kSteps; ++st) {
-      if (st == 0 || st < n_steps) {
+      if (kAll || st == 0 || st < n_steps) {
         uint32_t pf[2][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -370,7 +371,7 @@ bool make_short_map(CUtensorMap* map, const void* base, const FwdParams& p, cons
                         p.D >= 64 ? CU_TENSOR_MAP_SWIZZLE_128B : p.D == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-template <int D, int kKeys, bool kBf16>
+template <int D, int kKeys, bool kBf16, bool kAll>
 cudaError_t launch_short_one(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
   ShortPlan plan;
   plan.heads = p.B * p.H;
@@ -401,7 +402,7 @@ cudaError_t launch_short_one(const FwdParams& p, int sm_count, cudaStream_t stre
   const long long rounds = (plan.heads + grid * plan.teams - 1) / (grid * plan.teams);
   if (plan.stages > rounds) plan.stages = static_cast<int>(rounds);
   const int smem = plan.stages * stage_set + 1024;
-  auto kern = fwd_short_kernel<D, kKeys, kBf16>;
+  auto kern = fwd_short_kernel<D, kKeys, kBf16, kAll>;
   static std::atomic<unsigned long long> smem_done{0};   // per kernel instantiation, bit per device
   cudaError_t e = set_dynamic_smem_once(smem_done, reinterpret_cast<const void*>(kern), kRingBytesShort + 1024);
   if (e != cudaSuccess) return e;
@@ -410,13 +411,32 @@ cudaError_t launch_short_one(const FwdParams& p, int sm_count, cudaStream_t stre
   return e;
 }
 
+// Without the mask every row sees all steps: the loops over them have no branches then, and the score registers are
+// as many as the length needs, in steps of 32 keys (4096 heads, us: S = 100 D = 32 42.1 -> 40.1, S = 112 D = 16 33.4 ->
+// 29.5, S = 90 D = 64 46.1 -> 42.3, S = 20 D = 32, 8192 heads, 12.6 -> 11.9).  Not at D = 64 with 128 keys, where the
+// straight line spills (64.9 -> 66.8), and not with fewer than 64 keys' registers for causal rows of D >= 64 (S = 30
+// 21.9 -> 22.4).
+template <int D, int kKeys>
+cudaError_t launch_short_keys(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
+  if constexpr (D < 64 || kKeys < 128) {
+    if (!p.causal)
+      return p.bf16 ? launch_short_one<D, kKeys, true, true>(p, sm_count, stream, launches)
+                    : launch_short_one<D, kKeys, false, true>(p, sm_count, stream, launches);
+  }
+  return p.bf16 ? launch_short_one<D, kKeys, true, false>(p, sm_count, stream, launches)
+                : launch_short_one<D, kKeys, false, false>(p, sm_count, stream, launches);
+}
+
 template <int D>
 cudaError_t launch_short_dim(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
-  if (p.S <= 64)
-    return p.bf16 ? launch_short_one<D, 64, true>(p, sm_count, stream, launches)
-                  : launch_short_one<D, 64, false>(p, sm_count, stream, launches);
-  return p.bf16 ? launch_short_one<D, 128, true>(p, sm_count, stream, launches)
-                : launch_short_one<D, 128, false>(p, sm_count, stream, launches);
+  if (p.S <= 32 && (D < 64 || !p.causal)) return launch_short_keys<D, 32>(p, sm_count, stream, launches);
+  if (p.S <= 64) return launch_short_keys<D, 64>(p, sm_count, stream, launches);
+  if constexpr (D <= 64) {
+    if (p.S <= 96) return launch_short_keys<D, 96>(p, sm_count, stream, launches);
+    return launch_short_keys<D, 128>(p, sm_count, stream, launches);
+  } else {
+    return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace
@@ -430,8 +450,7 @@ cudaError_t launch_fwd_short(const FwdParams& p, int sm_count, cudaStream_t stre
     case 16: return launch_short_dim<16>(p, sm_count, stream, launches);
     case 32: return launch_short_dim<32>(p, sm_count, stream, launches);
     case 64: return launch_short_dim<64>(p, sm_count, stream, launches);
-    case 128: return p.bf16 ? launch_short_one<128, 64, true>(p, sm_count, stream, launches)
-                            : launch_short_one<128, 64, false>(p, sm_count, stream, launches);
+    case 128: return launch_short_dim<128>(p, sm_count, stream, launches);
     default: return cudaErrorInvalidValue;
   }
 }

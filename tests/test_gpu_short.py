@@ -31,7 +31,7 @@ def bound(v, dtype):
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_lengths_at_the_edges_of_strips_and_steps(fa, cuda_device, D, heads, dtype):
     B, H = heads
-    for S in (1, 15, 16, 17, 32, 33, 63, 64) + ((65, 97, 112, 113, 127, 128) if D <= 64 else ()):
+    for S in (1, 15, 16, 17, 31, 32, 33, 63, 64) + ((65, 95, 96, 97, 112, 113, 127, 128) if D <= 64 else ()):
         q, k, v = make_inputs(B, H, S, D, seed=S + D, dtype=dtype)
         for causal in (False, True):
             n0 = fa.launch_count()
