@@ -250,10 +250,19 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
     m_lo = fmaxf(m_lo, __shfl_xor_sync(0xffffffffu, m_lo, 2));
     m_hi = fmaxf(m_hi, __shfl_xor_sync(0xffffffffu, m_hi, 2));
 
+    // The maximum comes off before the scale goes on: exact where it counts, whatever the scores' size.  With s * scale -
+    // (m * scale) in one operation every P of the row is off by a factor 2^e, e the rounding error of m * scale; the
+    // division takes it out again, but from products of 2^28 (fp16) and 2^31 (fp32) on P does not hold it: rows whose
+    // keys a program hides with the type's lowest value came out as NaN.  The second operation costs 0 to 2 % (4096 heads,
+    // us: S = 100 D = 32 40.1 -> 40.5, S = 64 D = 64 23.1 -> 23.1, S = 128 D = 64 66.1 -> 67.5, S = 64 D = 128 49.5 -> 49.7);
+    // a branch for large rows only costs the same or more (the best form of it 7 % on S = 64 D = 128 causal).
+    // A row of nothing but -inf has the sum 0.
+    const float ref_lo = m_lo == -INFINITY ? 0.f : m_lo, ref_hi = m_hi == -INFINITY ? 0.f : m_hi;
+
     // ---- P = exp2((s - m) * scale), row sums, O += P V, step by step
     const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
-    const uint64_t neg_lo2 = pack_f32x2(-m_lo * scale_log2, -m_lo * scale_log2);
-    const uint64_t neg_hi2 = pack_f32x2(-m_hi * scale_log2, -m_hi * scale_log2);
+    const uint64_t neg_lo2 = pack_f32x2(-ref_lo, -ref_lo);
+    const uint64_t neg_hi2 = pack_f32x2(-ref_hi, -ref_hi);
     uint64_t sum_lo2 = pack_f32x2(0.f, 0.f), sum_hi2 = sum_lo2;
     float acc[D / 8][4];
 #pragma unroll
@@ -263,8 +272,8 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           float x0, x1, x2, x3;
-          unpack_f32x2(fma_f32x2(pack_f32x2(s[st][i][0], s[st][i][1]), scale2, neg_lo2), x0, x1);
-          unpack_f32x2(fma_f32x2(pack_f32x2(s[st][i][2], s[st][i][3]), scale2, neg_hi2), x2, x3);
+          unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(s[st][i][0], s[st][i][1]), neg_lo2), scale2), x0, x1);
+          unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(s[st][i][2], s[st][i][3]), neg_hi2), scale2), x2, x3);
           const float e0 = ex2(x0), e1 = ex2(x1), e2 = ex2(x2), e3 = ex2(x3);
           sum_lo2 = add_f32x2(sum_lo2, pack_f32x2(e0, e1));
           sum_hi2 = add_f32x2(sum_hi2, pack_f32x2(e2, e3));

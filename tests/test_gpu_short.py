@@ -81,3 +81,34 @@ def test_rows_with_infinite_scores_and_nan_stay_where_they_are(fa, cuda_device):
     bad = torch.isnan(ref).any(-1)
     assert torch.equal(torch.isnan(o).any(-1), bad) and bool(bad[0, 0, 5]) and int(bad.sum()) <= 2
     assert float((o - ref)[~bad].abs().max()) <= bound(v, torch.float16)
+
+
+def hidden_keys(S, D, dtype, hide, scale):
+    """Keys that a program hides with the type's lowest value (or -inf) in a column in which every query has a one,
+    or, `hide` = "none", scores of some 2^32 times the scale."""
+    q, k, v = make_inputs(2, 3, S, D, seed=S + D, dtype=dtype)
+    if hide == "none":
+        f = 2.0 ** 16 / scale ** 0.5
+        return (q.float() * f).to(dtype), (k.float() * f).to(dtype), v
+    q[..., 0] = 1.0
+    k[..., 0] = 0.0
+    first = {"front": S // 2, "all": S, "all, -inf": S}[hide]
+    k[:, :, :first, 0] = -math.inf if "inf" in hide else torch.finfo(dtype).min
+    return q, k, v
+
+
+@pytest.mark.parametrize("D", [16, 32, 64, 128])
+@pytest.mark.parametrize("hide", ["front", "all", "all, -inf", "none"])
+def test_scores_of_any_size(fa, cuda_device, D, hide):
+    # with the mask the first rows see hidden keys only; their softmax is over equal scores, not over nothing
+    for S in (20, 40, 64) + ((90, 128) if D <= 64 else ()):
+        scale = 1.0 / math.sqrt(D)
+        q, k, v = hidden_keys(S, D, torch.bfloat16, hide, scale)
+        for causal in (False, True):
+            o, lse = fa.attention_with_lse(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), causal, scale)
+            ref, lse_ref = attention_fp32(q, k, v, causal, scale, return_lse=True)
+            if "inf" in hide:   # a softmax over nothing
+                assert bool(torch.isnan(o).all()) and bool(torch.isneginf(lse).all())
+            else:
+                assert torch.allclose(lse.cpu(), lse_ref, atol=1e-4, rtol=1e-4), (S, causal)
+                assert float((o.cpu().float() - ref).abs().max()) <= bound(v, torch.bfloat16), (S, causal)
