@@ -651,7 +651,7 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
             mx[7] = max3(mx[7], __uint_as_float(s3[c + 2]), __uint_as_float(s3[c + 3]));
           }
           float mb = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7]));
-          if (mb == -INFINITY) mb = 0.f;  // only rows past S can get here; keep them finite
+          mb = fmaxf(mb, headroom * kLowestRef<kBf16>);   // a tile of nothing but hidden keys
           m_used = mb + headroom;
           if constexpr (kMode == kSplitKeys) {
             // the first PV of an item overwrites O_t: both groups must have read the last item's

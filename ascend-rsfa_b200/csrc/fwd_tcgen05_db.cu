@@ -536,7 +536,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
               mx[3] = max3(mx[3], __uint_as_float(s1[c + 2]), __uint_as_float(s1[c + 3]));
             }
             float mb = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
-            if (mb == -INFINITY) mb = 0.f;   // only rows past S can get here; keep them finite
+            mb = fmaxf(mb, headroom * kLowestRef<kBf16>);   // a tile of nothing but hidden keys
             m_used = mb + headroom;
           }
           RSFA_TRACE_EV(0x3000 + j);   // reference ready

@@ -30,6 +30,13 @@ constexpr float kHeadroomLog2 = RSFA_HEADROOM;
 // of it; all terms are non-negative) above which the softmax leaves its fast path; fp16 holds
 // 65504.
 constexpr float kSumLimit = RSFA_SUM_LIMIT;
+// Lowest reference a row can start with, in headrooms.  A first key tile whose scores are all hidden (-inf, or the type's
+// lowest value from a program that masks its keys that way) must leave a reference that the first visible tile lifts:
+// with one of 0 for -inf, visible scores below -2^7 or so were lost, and against the hidden scores themselves P is 2^e,
+// e the rounding error of score times scale: infinite, or zero.  2^29 and 2^32 (log2 units) are the first magnitudes
+// where 2^e leaves fp16 and bf16, so that no row which comes out right against its own maximum starts from here.
+template <bool kBf16>
+constexpr float kLowestRef = -(kBf16 ? 4294967296.f : 536870912.f) / kHeadroomLog2;
 
 // Wait-site tags (reported in the status word when a wait runs out).
 enum : int {

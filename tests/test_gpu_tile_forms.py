@@ -135,3 +135,28 @@ def test_storage_orders_agree_with_the_pair_kernel(fa, cuda_device, B, H, S, D):
             # each is within (2 u + S 2^-19) max|v| of the exact result (see agree)
             limit = 2 * (2 * u + S * 2.0 ** -19) * float(v.float().abs().max())
             assert float((o.float() - pair.float()).abs().max()) <= limit, (name, causal)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("hidden", ["lowest", "-inf"])
+@pytest.mark.parametrize("D,S,first,last", [(128, 640, 0, 128), (128, 640, 128, 256), (128, 640, 0, 256), (64, 384, 0, 64),
+                                            (64, 1000, 0, 128), (32, 300, 0, 64)])
+def test_a_first_key_tile_of_hidden_keys(fa, cuda_device, dtype, hidden, D, S, first, last):
+    # keys first .. last - 1 carry the type's lowest value (or -inf) in a column in which every query has a one; the
+    # visible scores lie around -8000 times the scale.  The first tile of a form's own keys may be hidden whole.
+    q, k, v = make_inputs(1, 3, S, D, seed=S + first, dtype=dtype)
+    q[..., :2] = 1.0
+    k[..., 0], k[..., 1] = 0.0, -8000.0
+    k[:, :, first:last, 0] = -math.inf if hidden == "-inf" else torch.finfo(dtype).min
+    scale = 1.0 / math.sqrt(D)
+    for causal in (False, True):
+        o, lse = fa.attention_with_lse(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), causal, scale)
+        torch.cuda.synchronize()
+        fa.device_status()
+        ref, lse_ref = attention_fp32(q, k, v, causal, scale, return_lse=True)
+        seen = slice(last if causal and first == 0 else 0, S)   # rows that see a visible key
+        u = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+        # as in agree(), and scores of 8000 are sums in fp32 whose order differs: 2 units of 2^-11 times the scale
+        limit = (2 * u + S * 2.0 ** -19 + 2.0 ** -10 * scale) * float(v.float().abs().max())
+        assert float((o.cpu().float() - ref)[:, :, seen].abs().max()) <= limit, causal
+        assert torch.allclose(lse.cpu()[:, :, seen], lse_ref[:, :, seen], atol=1e-3, rtol=1e-4), causal
