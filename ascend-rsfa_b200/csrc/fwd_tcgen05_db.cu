@@ -232,7 +232,13 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         // the WorkItem ring 1 to 4 % at D = 256, S = 1024 causal 330 -> 322 us, and 1 to 4 % at D <= 128).  Not
         // earlier: a CTA that claims far ahead of its need unbalances the end of the launch.  (D = 256 without
         // the mask: items all take equally long, and their Q is worth a whole item's head start.)
-        const int j_next = max(0, nmax - 4);
+        // And not before the last load where a few key tiles are most of an item: always with up to four, whose
+        // loads would wait for the queue, and up to S = 640 among the last two items per CTA, which are for the CTA
+        // that is free first (causal, us, early -> late: D = 256 S = 192 200 heads 20.5 -> 18.5, S = 100 4096 heads 143
+        // -> 129, S = 300 100 heads 20.5 -> 18.4; D = 128 S = 400 100 heads 18.1 -> 16.6; D = 64 S = 640 40 heads 12.4 ->
+        // 11.2.  Longer rows lose: D = 128 S = 768 148 heads 32.3 -> 34.5, D = 64 S = 1024 96 heads 27.6 -> 28.7).
+        const bool late = nmax <= 4 || (S <= 640 && cur.item >= sched.total_items - 2 * static_cast<int>(gridDim.x));
+        const int j_next = late ? nmax - 1 : nmax - 5;
         bool claimed = false;
         if (C::kQTmem && !p.causal) {
           next = claim();
@@ -270,13 +276,12 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         }
         ok = load_pair(&maps.k, 0, nmax > 1, 1, bar_kv_full((C::kJoint ? first_count++ : kv_count) % C::kStages));
         for (int j = 0; ok && j < nmax; ++j) {
-          if (j == j_next) {
-            if (!claimed) next = claim();
-            ok = publish(next);
-            if (!ok) break;
-          }
           ok = load_pair(&maps.v, j, j + 2 < nmax, j + 2,
                          C::kJoint ? bar_p_full(0, 0, step_count++) : bar_kv_full(kv_count % C::kStages));
+          if (ok && j == j_next) {
+            if (!claimed) next = claim();
+            ok = publish(next);
+          }
         }
       }
     }

@@ -160,3 +160,23 @@ def test_a_first_key_tile_of_hidden_keys(fa, cuda_device, dtype, hidden, D, S, f
         limit = (2 * u + S * 2.0 ** -19 + 2.0 ** -10 * scale) * float(v.float().abs().max())
         assert float((o.cpu().float() - ref)[:, :, seen].abs().max()) <= limit, causal
         assert torch.allclose(lse.cpu()[:, :, seen], lse_ref[:, :, seen], atol=1e-3, rtol=1e-4), causal
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D,S,heads", [(256, 64, 700), (256, 130, 400), (256, 256, 300), (256, 640, 70), (128, 320, 300),
+                                       (128, 640, 120), (64, 200, 500), (64, 641, 160)])
+def test_work_items_of_one_to_eleven_key_tiles_on_the_64_key_kernels(fa, cuda_device, D, S, heads, causal):
+    # where the producer claims its next item: items of up to four tiles, and the last ones of a short-row launch
+    g = torch.Generator(device=cuda_device).manual_seed(S)
+    q, k, v = [torch.randn(heads, 1, S, D, generator=g, device=cuda_device).half() for _ in range(3)]
+    o = fa.attention(q, k, v, causal, 1.0 / math.sqrt(D), 128, 64)
+    fa.set_option("force_path", 0)
+    try:
+        general = fa.attention(q, k, v, causal, 1.0 / math.sqrt(D), 128, 64)
+    finally:
+        fa.set_option("force_path", -1)
+    torch.cuda.synchronize()
+    fa.device_status()
+    # each is within (2 u + S 2^-19) max|v| of the exact result (see agree)
+    limit = 2 * (2 * 2.0 ** -11 + S * 2.0 ** -19) * float(v.float().abs().max())
+    assert float((o.float() - general.float()).abs().max()) <= limit
