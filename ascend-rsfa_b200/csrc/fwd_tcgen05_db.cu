@@ -179,6 +179,11 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
   griddep_wait();
 
   const int S = p.S;
+  auto load_q_tile = [&](int t, const WorkItem& w) {
+    mbar_arrive_expect_tx(bar_q_full(t), C::kQTileBytes);
+    for (int bx = 0; bx < C::kBoxes; ++bx)
+      tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64, w.row0 + t * kRowsDb, w.h, w.b);
+  };
   if (warp == C::kTmaWarp) {
     // ================================================================ producer
     if (lane == 0) {
@@ -221,6 +226,12 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         return true;
       };
       WorkItem next = claim();
+      if constexpr (C::kQWarp) {
+        // The first item's Q from here: handed over to its loader it starts 300 clk later, which a launch of one item
+        // per CTA has nothing to hide behind (us: D = 128 causal 74 heads of S = 400 14.1 -> 13.7, 100 of S = 200 10.5 ->
+        // 10.2; D = 64 causal 66 heads of S = 384 9.8 -> 9.5).
+        for (int t = 0; t < NT; ++t) load_q_tile(t, next);
+      }
       ok = publish(next);
       while (ok && next.item < sched.total_items) {
         const WorkItem cur = next;
@@ -297,13 +308,9 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         const WorkItem w = ring_get(sched_ring + 16u * slot);
         mbar_arrive(bar_sched_empty0 + 8u * slot);
         if (w.item >= sched.total_items) break;
-        for (int t = 0; ok && t < NT; ++t) {
+        for (int t = 0; ok && item_count > 0 && t < NT; ++t) {   // the first item's is under way
           ok = mbar_wait(bar_q_empty(t), (item_count & 1) ^ 1, abort_flag, wait_ns, kTagQEmpty);
-          if (!ok) break;
-          mbar_arrive_expect_tx(bar_q_full(t), C::kQTileBytes);
-          for (int bx = 0; bx < C::kBoxes; ++bx)
-            tma_load_4d(sQ + t * C::kQTileBytes + bx * C::kQBoxBytes, &maps.q, bar_q_full(t), bx * 64, w.row0 + t * kRowsDb,
-                        w.h, w.b);
+          if (ok) load_q_tile(t, w);
         }
         ++item_count;
       }
