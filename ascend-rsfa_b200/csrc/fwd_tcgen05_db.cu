@@ -735,16 +735,21 @@ cudaError_t launch_db(const FwdParams& p, int sm_count, cudaStream_t stream, lon
 // work-item boundaries (last PV, epilogue, first QK^T: 3000 to 5000 clk, as long as two to three key tiles) and
 // deal out 128 rows at a time, where a pair ends when its longer tile does; but each loads its own K/V tiles and
 // a step is only 64 keys, so long rows in plenty are better off with the separate-P kernel (128 keys, K/V shared).
-// Measured at D = 64, best pair kernel -> this, us: S = 200 128 heads x 1000 / 128 36.5 -> 34.6, 300 heads 16.9 ->
-// 15.2; S = 384 1000 heads 75.2 -> 61.4, causal 59.0 -> 49.1; S = 512 causal 128 heads 15.3 -> 14.4, 1000 heads
-// 78.2 -> 74.6; S = 1024 causal 12 heads 17.0 -> 13.7, 1000 heads 229.6 -> 225.4; S = 2048 causal 12 heads 28.7 ->
-// 22.4, 48 heads 43.7 -> 42.8.  Beyond the lines drawn here it loses: S = 1024 300 heads 111 -> 115, S = 2048 167 ->
-// 180, causal S = 2048 128 heads 101.6 -> 104.2, S = 3000 40 heads 70.1 -> 70.9; causal S <= 160 (a second tile of a few rows) 25.8 -> 26.5, and causal
-// S <= 256 when pairs fill one wave but single tiles need second places on the SMs, 7.5 -> 8.2.
+// Measured at D = 64, best pair kernel -> this, us: S = 200 1000 heads 38.2 -> 34.8, 300 heads 17.6 -> 15.0; S = 384
+// 1000 heads 75.8 -> 61.9, causal 61.7 -> 50.2; S = 512 causal 128 heads 16.3 -> 15.1, 1000 heads 82.5 -> 75.2;
+// S = 1024 causal 12 heads 17.1 -> 14.1, 1000 heads 255 -> 246; S = 2048 causal 12 heads 28.7 -> 22.4, 48 heads 45.7 ->
+// 45.7.  Beyond the lines drawn here it loses: S = 1024 300 heads 111 -> 115, S = 2048 167 -> 180, causal S = 2048 128
+// heads 101.6 -> 104.2, S = 3000 40 heads 70.1 -> 70.9; S = 449 to 512, whose keys fill the pair's 128-key tiles, from
+// 4000 tiles on, where the second reading of K and V tells (4096 heads 451 -> 458; 1000 heads 111 -> 111; S = 448 wins at
+// any size, 4096 heads 453 -> 392); causal S <= 160 (a second tile of a few rows) 25.8 -> 26.5, and causal S <= 320 when
+// pairs fill one wave but single tiles need second places on the SMs (66 heads of S = 320 8.7 -> 9.2, 60 of S = 257 8.4 ->
+// 8.9, 148 of S = 256 7.5 -> 8.2).
 bool single_tiles_pay(const FwdParams& p, int sm_count) {
-  const long long tiles = static_cast<long long>(p.B) * p.H * ((p.S + kRowsDb - 1) / kRowsDb);
-  if (!p.causal) return p.S <= 512 || (p.S <= 1024 && tiles <= 13ll * sm_count);
-  if (p.S <= 256 && tiles > sm_count) return p.S > 160 && tiles > 2 * sm_count;
+  const long long heads = static_cast<long long>(p.B) * p.H;
+  const long long tiles = heads * ((p.S + kRowsDb - 1) / kRowsDb), pairs = heads * ((p.S + 2 * kRowsDb - 1) / (2 * kRowsDb));
+  if (!p.causal) return p.S <= 448 || (p.S <= 1024 && tiles <= (p.S <= 512 ? 27ll : 13ll) * sm_count);
+  if (p.S <= 160 && tiles > sm_count) return false;
+  if (p.S <= 320 && pairs <= sm_count && tiles > sm_count) return false;
   return p.S <= 1024 || tiles <= 5ll * sm_count;
 }
 
