@@ -13,8 +13,9 @@ return types —
 sm_100a kernels in librsfa_b200.so, reached through its C ABI - from a small
 native extension for the ordinary call, with ctypes for the rest; this file only
 validates, allocates the output like the reference does (``torch.empty_like(q)``,
-:558) and passes raw pointers, strides and the current CUDA stream.  There is no Triton, no PyTorch math and no CPU path here: without
-the library, or on a non-CUDA tensor, the call raises.
+:558) and passes raw pointers, strides and the current CUDA stream.  There is no
+Triton, no PyTorch math and no CPU path here: without the library, or on a non-CUDA
+tensor, the call raises.
 
 Differences from the reference, all on purpose:
 * BLOCK_M / BLOCK_N are a request.  Results never depend on them (true of the
@@ -26,19 +27,23 @@ Differences from the reference, all on purpose:
   the log-sum-exp (the reference writes it on the non-causal path only, :400-404).
 """
 import ctypes
+import warnings
 
 import torch
 
 from . import _capi
 
+_lib = _capi.load()
+
 try:
     from . import _rsfa_torch
-except ImportError as e:
-    raise ImportError("the PyTorch side of the operator call is not built for this torch: run "
-                      "`python ascend-rsfa_b200/build.py` (%s)" % e) from e
 
-_lib = _capi.load()
-_rsfa_torch.bind(ctypes.cast(_lib.rsfa_fwd, ctypes.c_void_p).value)
+    _rsfa_torch.bind(ctypes.cast(_lib.rsfa_fwd, ctypes.c_void_p).value)
+except ImportError as e:
+    # the same kernels through ctypes
+    warnings.warn("the native form of the attention() call is not in use (%s): calls cost 10 us more of host time; "
+                  "`python ascend-rsfa_b200/build.py` builds it" % e, RuntimeWarning)
+    _rsfa_torch = None
 
 DEVICE = "cuda"
 _DTYPES = {torch.float16: _capi.RSFA_DTYPE_F16, torch.bfloat16: _capi.RSFA_DTYPE_BF16}
@@ -94,7 +99,7 @@ def _dense(t):
 def _forward(q, k, v, causal, sm_scale, BM, BN, want_lse):
     # The ordinary call - dense CUDA tensors on the current device, plain argument types, no modes or
     # transforms - in native code, 10 us of Python less (csrc/torch_binding.cpp); None: not ordinary.
-    done = _rsfa_torch.forward(q, k, v, causal, sm_scale, BM, BN, want_lse)
+    done = None if _rsfa_torch is None else _rsfa_torch.forward(q, k, v, causal, sm_scale, BM, BN, want_lse)
     if type(done) is tuple:
         return done
     if done is not None:

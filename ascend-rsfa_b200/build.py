@@ -3,7 +3,9 @@
     python ascend-rsfa_b200/build.py [--force] [--verbose] [--trace]
 
 Beside the library, the PyTorch side of the operator call (csrc/torch_binding.cpp) is
-compiled against the installed torch into ascend_rsfa/_rsfa_torch*.so.
+compiled against the installed torch into ascend_rsfa/_rsfa_torch*.so.  The library needs
+no torch and is built without one; so does attention() run without the extension, 10 us
+of host time slower.
 
 The library lands beside the Python module that loads it
 (ascend_rsfa/librsfa_b200.so) together with a stamp file holding a hash of the
@@ -39,39 +41,60 @@ FLAGS = [
 
 BINDING = "torch_binding.cpp"
 OUT_BINDING = os.path.join(HERE, "ascend_rsfa", "_rsfa_torch" + sysconfig.get_config_var("EXT_SUFFIX"))
+BINDING_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
+# what the extension is made from, beside the torch and the Python it is compiled against
+BINDING_INPUTS = [os.path.join(CSRC, BINDING)]
 
 
-def binding_command():
-    """The g++ command line of the PyTorch extension: headers and libraries of the torch in use."""
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+def torch_home():
+    """Directory of the installed torch, or None: no torch, or one without CUDA, which has no tensor to call with."""
+    spec = importlib.util.find_spec("torch")
+    if spec is None or spec.origin is None:
+        return None
+    home = os.path.dirname(spec.origin)
+    return home if os.path.exists(os.path.join(home, "lib", "libc10_cuda.so")) else None
+
+
+def binding_command(home):
+    """The g++ command line of the PyTorch extension: headers, libraries and C++ ABI of the torch in use."""
+    import torch
+
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
-    inc = [sysconfig.get_paths()["include"], os.path.join(torch_dir, "include"),
-           os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
-    lib = os.path.join(torch_dir, "lib")
-    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1"] +
-            ["-I" + i for i in inc] + [os.path.join(CSRC, BINDING), "-o", OUT_BINDING, "-L" + lib] +
+    inc = [sysconfig.get_paths()["include"], os.path.join(home, "include"),
+           os.path.join(home, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+    return (["g++"] + BINDING_FLAGS +
+            ["-D_GLIBCXX_USE_CXX11_ABI=%d" % torch.compiled_with_cxx11_abi()] +
+            ["-I" + i for i in inc] + [os.path.join(CSRC, BINDING), "-o", OUT_BINDING, "-L" + os.path.join(home, "lib")] +
             ["-l" + n for n in ("torch_python", "torch", "torch_cpu", "c10_cuda", "c10")])
 
 
-def binding_hash():
-    """Hash of the extension's source, its command line and the torch and Python it is built against."""
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+def binding_hash(home):
+    """Hash of the extension's sources and flags and of the torch and Python it is built against; no paths, so that a
+    tree that moves to another machine with the same torch stays as it is."""
     h = hashlib.sha256()
-    for f in (os.path.join(CSRC, BINDING), os.path.join(torch_dir, "version.py")):
+    for f in BINDING_INPUTS + [os.path.join(home, "version.py")]:
         with open(f, "rb") as fh:
             h.update(fh.read() + b"\0")
-    h.update(" ".join(binding_command()).encode() + sys.version.encode())
+    h.update(" ".join(BINDING_FLAGS).encode() + sys.version.encode())
     return h.hexdigest()
 
 
 def build_binding(force=False):
+    """The extension, or None where there is nothing to build it with: attention() then takes the ctypes route."""
+    home = torch_home()
+    if home is None:
+        sys.stderr.write("no torch with CUDA here: %s is not built\n" % os.path.basename(OUT_BINDING))
+        return None
     stamp = OUT_BINDING + ".stamp"
-    want = binding_hash()
+    want = binding_hash(home)
     if not force and os.path.exists(OUT_BINDING) and os.path.exists(stamp):
         with open(stamp) as fh:
             if fh.read().strip() == want:
                 return OUT_BINDING
-    r = subprocess.run(binding_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if shutil.which("g++") is None:
+        sys.stderr.write("no g++ here: %s is not built\n" % os.path.basename(OUT_BINDING))
+        return None
+    r = subprocess.run(binding_command(home), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError("g++ failed on " + BINDING)
@@ -106,9 +129,15 @@ def stale(out, flags):
 
 
 def build(force=False, verbose=False, trace=False):
+    out = build_library(force, verbose, trace)
+    if not trace:
+        build_binding(force)
+    return out
+
+
+def build_library(force=False, verbose=False, trace=False):
     out = OUT_TRACE if trace else OUT
     flags = FLAGS + (["-DRSFA_TRACE"] if trace else [])
-    build_binding(force)
     if not force and not stale(out, flags):
         return out
     nvcc = find_nvcc()
