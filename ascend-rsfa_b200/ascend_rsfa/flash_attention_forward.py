@@ -38,6 +38,9 @@ _lib = _capi.load()
 try:
     from . import _rsfa_torch
 
+    _built_for = getattr(_rsfa_torch, "torch_version", "an unnamed version")
+    if _built_for != str(torch.__version__):
+        raise ImportError("built for torch %s, this is %s" % (_built_for, torch.__version__))
     _rsfa_torch.bind(ctypes.cast(_lib.rsfa_fwd, ctypes.c_void_p).value)
 except ImportError as e:
     # the same kernels through ctypes

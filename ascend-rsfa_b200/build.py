@@ -22,6 +22,7 @@ under profiles/ come from that build; the product library has no trace code.
 import hashlib
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -43,7 +44,7 @@ BINDING = "torch_binding.cpp"
 OUT_BINDING = os.path.join(HERE, "ascend_rsfa", "_rsfa_torch" + sysconfig.get_config_var("EXT_SUFFIX"))
 BINDING_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
 # what the extension is made from, beside the torch and the Python it is compiled against
-BINDING_INPUTS = [os.path.join(CSRC, BINDING)]
+BINDING_INPUTS = [os.path.join(CSRC, BINDING), os.path.join(HERE, "..", "include", "rsfa.h")]
 
 
 def torch_home():
@@ -55,6 +56,11 @@ def torch_home():
     return home if os.path.exists(os.path.join(home, "lib", "libc10_cuda.so")) else None
 
 
+def torch_version(home):
+    with open(os.path.join(home, "version.py")) as fh:
+        return re.search(r"^__version__ = ['\"]([^'\"]+)['\"]", fh.read(), re.M).group(1)
+
+
 def binding_command(home):
     """The g++ command line of the PyTorch extension: headers, libraries and C++ ABI of the torch in use."""
     import torch
@@ -63,7 +69,8 @@ def binding_command(home):
     inc = [sysconfig.get_paths()["include"], os.path.join(home, "include"),
            os.path.join(home, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
     return (["g++"] + BINDING_FLAGS +
-            ["-D_GLIBCXX_USE_CXX11_ABI=%d" % torch.compiled_with_cxx11_abi()] +
+            ["-D_GLIBCXX_USE_CXX11_ABI=%d" % torch.compiled_with_cxx11_abi(),
+             '-DRSFA_TORCH_VERSION="%s"' % torch_version(home)] +
             ["-I" + i for i in inc] + [os.path.join(CSRC, BINDING), "-o", OUT_BINDING, "-L" + os.path.join(home, "lib")] +
             ["-l" + n for n in ("torch_python", "torch", "torch_cpu", "c10_cuda", "c10")])
 

@@ -18,11 +18,12 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include "../../include/rsfa.h"
+
 namespace {
 
 // rsfa_fwd of the library that the Python side has loaded (bind() hands its address over).
-using FwdFn = int (*)(const void*, const void*, const void*, void*, float*, int, int, int, int, const int64_t*, int,
-                      float, int, int, int, void*);
+using FwdFn = decltype(&rsfa_fwd);
 FwdFn g_fwd = nullptr;
 
 bool plain_mode() {
@@ -99,7 +100,7 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   float* lp = lse.defined() ? static_cast<float*>(lse.mutable_data_ptr()) : nullptr;
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
   const float scale = static_cast<float>(PyFloat_AS_DOUBLE(args[4]));
-  const int dtype = q.scalar_type() == at::kBFloat16 ? 1 : 0;
+  const int dtype = q.scalar_type() == at::kBFloat16 ? RSFA_DTYPE_BF16 : RSFA_DTYPE_F16;
   const int B = static_cast<int>(q.size(0)), H = static_cast<int>(q.size(1)), S = static_cast<int>(q.size(2));
   const int causal = args[3] == Py_True ? 1 : 0;
   int rc = 0;
@@ -148,4 +149,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_rsfa_torch", nullptr, -1, methods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__rsfa_torch() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__rsfa_torch() {
+  PyObject* m = PyModule_Create(&module);
+  // the torch whose tensor layout this file was compiled for: the Python side uses it with no other
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", RSFA_TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}

@@ -1,12 +1,14 @@
 """What build.py needs for what, and what the operator module does without the native form of its call."""
 import importlib.util
 import os
+import re
 import subprocess
 import sys
 
 import pytest
+import torch
 
-from conftest import PKG
+from conftest import PKG, ROOT
 
 
 @pytest.fixture
@@ -66,11 +68,38 @@ def test_the_library_comes_first(fresh, monkeypatch):
     assert order == ["library", "binding", "library"]
 
 
+def test_the_extension_is_stale_when_the_c_interface_or_torch_changes(build, tmp_path, monkeypatch):
+    home = build.torch_home()
+    before = build.binding_hash(home)
+    assert os.path.join(ROOT, "include", "rsfa.h") in [os.path.abspath(f) for f in build.BINDING_INPUTS]
+    header = tmp_path / "rsfa.h"
+    header.write_text("changed")
+    monkeypatch.setattr(build, "BINDING_INPUTS", build.BINDING_INPUTS[:-1] + [str(header)])
+    assert build.binding_hash(home) != before
+    monkeypatch.undo()
+    monkeypatch.setattr(build, "find_nvcc", missing)
+    assert build.binding_hash(home) == before                     # where nvcc lies is no part of it
+    (tmp_path / "version.py").write_text("__version__ = '0.1'\n")
+    assert build.binding_hash(str(tmp_path)) != before and build.torch_version(str(tmp_path)) == "0.1"
+
+
+def test_the_extension_takes_the_signature_from_the_header():
+    text = open(os.path.join(PKG, "csrc", "torch_binding.cpp")).read()
+    assert '#include "../../include/rsfa.h"' in text and re.search(r"using FwdFn = decltype\(&rsfa_fwd\)", text)
+
+
 IMPORT = """
-import sys, warnings
+import sys, types, warnings
 sys.path.insert(0, %r)
 import torch
-sys.modules["ascend_rsfa._rsfa_torch"] = None
+if %r == "missing":
+    sys.modules["ascend_rsfa._rsfa_torch"] = None
+else:
+    m = types.ModuleType("ascend_rsfa._rsfa_torch")
+    if %r == "older":
+        m.torch_version = "1.0"
+    m.bind = m.forward = lambda *a: 1 / 0
+    sys.modules["ascend_rsfa._rsfa_torch"] = m
 with warnings.catch_warnings(record=True) as seen:
     warnings.simplefilter("always")
     import ascend_rsfa.flash_attention_forward as fa
@@ -85,6 +114,14 @@ except RuntimeError as e:
 """
 
 
-def test_the_operator_runs_without_the_extension():
-    r = subprocess.run([sys.executable, "-c", IMPORT % PKG], capture_output=True, text=True, timeout=300)
+@pytest.mark.parametrize("extension", ["missing", "older", "without a version"])
+def test_the_operator_runs_without_the_extension(extension):
+    """Not built, or built for another torch, whose tensors may be laid out differently: the ctypes route."""
+    r = subprocess.run([sys.executable, "-c", IMPORT % (PKG, extension, extension)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "python-route-ok (128, 128)" in r.stdout, r.stdout + r.stderr
+
+
+def test_the_extension_in_use_was_built_for_this_torch():
+    import ascend_rsfa.flash_attention_forward as fa
+
+    assert fa._rsfa_torch is not None and fa._rsfa_torch.torch_version == str(torch.__version__)
