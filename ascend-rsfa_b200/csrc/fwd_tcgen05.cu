@@ -1044,7 +1044,9 @@ extern "C" int rsfa_fwd_noalloc(const void* q, const void* k, const void* v, voi
   }
   // Only the tcgen05 kernel uses scratch; shapes it is not built for have no variant here.
   if (!tcgen05_supports(S, D, sm_scale)) return RSFA_ERR_UNSUPPORTED;
-  const int rows_per_item = (D == 256) ? kTileM : kNT * kTileM;   // both families use 256-row items at D <= 128
+  // In items of 256 rows at D <= 128.  The forms with 128-row items are not chosen where they would be more than 2^30
+  // of those (single_tiles_pay; split_keys_pays stops at 16 per multiprocessor).
+  const int rows_per_item = (D == 256) ? kTileM : kNT * kTileM;
   const long long items = static_cast<long long>(B) * H * ((S + rows_per_item - 1) / rows_per_item);
   if (items > kNoAllocMaxItems) return RSFA_ERR_TOO_LARGE;
 

@@ -747,6 +747,7 @@ cudaError_t launch_db(const FwdParams& p, int sm_count, cudaStream_t stream, lon
 bool single_tiles_pay(const FwdParams& p, int sm_count) {
   const long long heads = static_cast<long long>(p.B) * p.H;
   const long long tiles = heads * ((p.S + kRowsDb - 1) / kRowsDb), pairs = heads * ((p.S + 2 * kRowsDb - 1) / (2 * kRowsDb));
+  if (tiles > (1ll << 30)) return false;   // work items are numbered in 32 bits, and callers may bring 2^30 pairs
   if (!p.causal) return p.S <= 448 || (p.S <= 1024 && tiles <= (p.S <= 512 ? 27ll : 13ll) * sm_count);
   if (p.S <= 160 && tiles > sm_count) return false;
   if (p.S <= 320 && pairs <= sm_count && tiles > sm_count) return false;
