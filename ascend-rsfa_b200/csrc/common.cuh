@@ -31,8 +31,8 @@ struct FwdParams {
   unsigned long long wait_limit_ns;
   int pdl;             // 1: launch with programmatic stream serialisation (the "pdl" option)
   // Test hook (the "test_drop_load" option, -1 = off): the producer of the 128-key tcgen05 kernel
-  // leaves out its n-th K/V tile load together with the barrier arrival that announces it.  Nothing
-  // is in flight for that tile and no address is touched; the consumer's bounded wait simply runs
+  // leaves out its n-th K/V tile load together with the barrier arrival that announces it, and the kernel
+  // for a single key tile the loads of head n.  Nothing is in flight for that tile and no address is touched; the consumer's bounded wait simply runs
   // out, which is how the tests reach the wait-expired path on a healthy GPU.
   int test_drop_load;
 #ifdef RSFA_TRACE
@@ -60,7 +60,7 @@ cudaError_t launch_fwd_generic(const FwdParams& p, cudaStream_t stream, long lon
 long long generic_grid_blocks(int B, int H, int S);
 cudaError_t launch_fwd_tcgen05(const FwdParams& p, int sm_count, cudaStream_t stream,
                                long long* launches);
-// The single-key-tile kernel (fwd_short.cu), S <= 128 and D <= 64.
+// The single-key-tile kernel (fwd_short.cu), S <= 128 at D <= 64 and S <= 64 at D = 128.
 cudaError_t launch_fwd_short(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches);
 bool short_fits(int S, int D, float sm_scale);
 // The double-buffered-S family (D = 64, 128, 256), selected by launch_fwd_tcgen05.

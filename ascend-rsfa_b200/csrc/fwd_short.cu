@@ -149,6 +149,7 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
   };
   // one lane: Q, K and V of head `bh` into a slot of this team
   auto load_head = [&](int bh, int slot) {
+    if (bh == p.test_drop_load) return;   // test hook: this head is never announced
     const uint32_t bar = smem_u32(&full_bar[team * plan.stages + slot]);
     const uint32_t dst = ring + slot * slot_bytes;
     const int b = batch_of(bh), h = bh - b * p.H;

@@ -1,6 +1,7 @@
 """The single-key-tile kernel (csrc/fwd_short.cu) on a B200: edges of its strips of 16 rows, its steps of 32
 keys and its ring plan, every head dimension it takes, against the fp32 oracle; storage orders against the
 general mma.sync kernel."""
+import ctypes
 import math
 
 import pytest
@@ -112,3 +113,31 @@ def test_scores_of_any_size(fa, cuda_device, D, hide):
             else:
                 assert torch.allclose(lse.cpu(), lse_ref, atol=1e-4, rtol=1e-4), (S, causal)
                 assert float((o.cpu().float() - ref).abs().max()) <= bound(v, torch.bfloat16), (S, causal)
+
+
+@pytest.mark.parametrize("B,H,S,D,head", [(5, 6, 100, 64, 7), (400, 4, 64, 128, 1599), (3000, 4, 16, 16, 11000)])
+def test_a_wait_that_runs_out_is_reported(fa, cuda_device, B, H, S, D, head):
+    """The loads of one head and the arrival that announces them are left out ("test_drop_load"): nothing is in flight and
+    no address is touched, the wait of the team that owns the head runs out and the kernel returns by itself."""
+    from ascend_rsfa import _capi
+
+    lib = _capi.load()
+    q, k, v = [t.to(cuda_device) for t in make_inputs(B, H, S, D, seed=8)]
+    whole = fa.attention(q, k, v, False, 0.2, 64, 64)
+    fa.device_status()
+    fa.set_option("wait_limit_ms", 1)
+    fa.set_option("test_drop_load", head)     # the first head of a team, and ones that go to slots used before
+    try:
+        fa.attention(q, k, v, False, 0.2, 64, 64)
+        torch.cuda.synchronize()
+    finally:
+        fa.set_option("test_drop_load", -1)
+        fa.set_option("wait_limit_ms", 2000)
+    raw = ctypes.c_int(0)
+    assert lib.rsfa_device_status(0, ctypes.byref(raw)) == _capi.RSFA_ERR_DEVICE_STATUS
+    assert raw.value == (1 << 16) | 4, hex(raw.value)     # the wait for K/V
+    for _ in range(2):
+        o = fa.attention(q, k, v, False, 0.2, 64, 64)
+        torch.cuda.synchronize()
+        assert torch.equal(o, whole)
+    fa.device_status()
