@@ -47,6 +47,12 @@ struct DbCfg {
   // One Q tile at D <= 64 needs half of everything (192 tensor-memory columns, 97 KB): two CTAs per SM.
   static constexpr int kCtasPerSm = (NT == 1 && D != 256) ? 2 : 1;
   static constexpr int kTmemCols = 512 / kCtasPerSm;
+  // The one-tile form takes a row's reference from the keys of the tile that was asked for, 128 or 64, as the kernel of
+  // that tile does.  The row's largest weight is a power of two, and exact in 16 bits, when it is among them: from 64
+  // keys where it had been 128, the error against 64-bit sums was 1.6 % larger on average (S = 129 to 1024, scores of 1 to
+  // 6 log2 units), 17 % at S = 132.  The look at the second tile costs an item some 300 clk (without the mask, us: 300 heads
+  // of S = 200 14.7 -> 15.7, 1000 of S = 384 65.2 -> 66.4, 128 of S = 1024 51.2 -> 52.1).
+  static constexpr bool kRefAhead = (kCtasPerSm == 2);
   // One Q tile: the bytes of the ring entry that a step needs, (V_j, K_{j+2}), are counted on the barrier on which
   // the softmax hands over P_j, so the MMA warp waits once per step.  The loads run up to kStages entries ahead of
   // the softmax: kTurns such barriers are used in turn (kTurns >= kStages: a barrier's turn comes again when the
@@ -505,6 +511,37 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
       // says that a P value might leave the 16-bit range is that tile redone by
       // softmax_half_careful, which moves the reference and rescales this thread's row of O_t.
       float m_used = -INFINITY;   // reference, raw score units
+      if constexpr (C::kRefAhead) {
+        if (p.tile_n == 2 * kKeysDb && n > 1) {   // both S buffers are filled before the first hand-over of P
+          ok = mbar_wait_warp(bar_s_full(t, 1), s_count[1] & 1, abort_flag, wait_ns, kTagSFull);
+          if (!ok) break;
+          tc_fence_after_sync();
+          uint32_t a[32], b[32];
+          tmem_ld_x32(tmem_base + lane_base + C::col_s(t, 1), a);
+          tmem_ld_x32(tmem_base + lane_base + C::col_s(t, 1) + 32, b);
+          tmem_wait_ld();
+          reg_fence_x32(a);
+          reg_fence_x32(b);
+          int limit = S - 1 - kKeysDb;            // last visible column of the second key tile
+          if (p.causal) limit = min(limit, row - kKeysDb);
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          auto seen = [&](uint32_t v, int c) { return c > limit ? -INFINITY : __uint_as_float(v); };
+          if (__any_sync(0xffffffffu, limit < kKeysDb - 1)) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) {
+              mx[c & 2] = max3(mx[c & 2], seen(a[c], c), seen(a[c + 1], c + 1));
+              mx[(c & 2) + 1] = max3(mx[(c & 2) + 1], seen(b[c], c + 32), seen(b[c + 1], c + 33));
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) {
+              mx[c & 2] = max3(mx[c & 2], __uint_as_float(a[c]), __uint_as_float(a[c + 1]));
+              mx[(c & 2) + 1] = max3(mx[(c & 2) + 1], __uint_as_float(b[c]), __uint_as_float(b[c + 1]));
+            }
+          }
+          m_used = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+        }
+      }
       float l = 0.f;
       int j = 0;
       while (j < n) {
@@ -547,7 +584,7 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
               mx[2] = max3(mx[2], __uint_as_float(s1[c]), __uint_as_float(s1[c + 1]));
               mx[3] = max3(mx[3], __uint_as_float(s1[c + 2]), __uint_as_float(s1[c + 3]));
             }
-            float mb = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+            float mb = max3(max3(mx[0], mx[1], mx[2]), mx[3], m_used);   // m_used: the second tile's maximum, or -inf
             mb = fmaxf(mb, headroom * kLowestRef<kBf16>);   // a tile of nothing but hidden keys
             m_used = mb + headroom;
           }
@@ -642,8 +679,9 @@ fwd_tcgen05_db_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, c
         store_o_rows<D, kBf16, C::kStageBufs>(tO, inv_l, sStage + t * C::kStageBytes + wq * (4096 * C::kStageBufs), lane,
                                               &maps.o, tile_row0 + wq * 32, h, b, tile_row0 + wq * 32 < S);
       }
+      // from the product that P was taken against, rounding and all: the factor it puts on l then drops out
       if (p.lse != nullptr && row < S)
-        p.lse[(static_cast<int64_t>(w.b) * p.H + w.h) * S + row] = m_used * p.sm_scale + logf(l);
+        p.lse[(static_cast<int64_t>(w.b) * p.H + w.h) * S + row] = m_used * scale_log2 * kLn2 + logf(l);
       tc_fence_before_sync();
       RSFA_TRACE_EV(0x7000);   // epilogue done
     }
