@@ -773,15 +773,17 @@ cudaError_t launch_db(const FwdParams& p, int sm_count, cudaStream_t stream, lon
 // work-item boundaries (last PV, epilogue, first QK^T: 3000 to 5000 clk, as long as two to three key tiles) and
 // deal out 128 rows at a time, where a pair ends when its longer tile does; but each loads its own K/V tiles and
 // a step is only 64 keys, so long rows in plenty are better off with the separate-P kernel (128 keys, K/V shared).
-// Measured at D = 64, best pair kernel -> this, us: S = 200 1000 heads 38.2 -> 34.8, 300 heads 17.6 -> 15.0; S = 384
-// 1000 heads 75.8 -> 61.9, causal 61.7 -> 50.2; S = 512 causal 128 heads 16.3 -> 15.1, 1000 heads 82.5 -> 75.2;
-// S = 1024 causal 12 heads 17.1 -> 14.1, 1000 heads 255 -> 246; S = 2048 causal 12 heads 28.7 -> 22.4, 48 heads 45.7 ->
-// 45.7.  Beyond the lines drawn here it loses: S = 1024 300 heads 111 -> 115, S = 2048 167 -> 180, causal S = 2048 128
-// heads 101.6 -> 104.2, S = 3000 40 heads 70.1 -> 70.9; S = 449 to 512, whose keys fill the pair's 128-key tiles, from
-// 4000 tiles on, where the second reading of K and V tells (4096 heads 451 -> 458; 1000 heads 111 -> 111; S = 448 wins at
-// any size, 4096 heads 453 -> 392); causal S <= 160 (a second tile of a few rows) 25.8 -> 26.5, and causal S <= 320 when
-// pairs fill one wave but single tiles need second places on the SMs (66 heads of S = 320 8.7 -> 9.2, 60 of S = 257 8.4 ->
-// 8.9, 148 of S = 256 7.5 -> 8.2).
+// Measured at D = 64, best pair kernel -> this, us: S = 200 1000 heads 38.3 -> 36.9, 300 heads 17.5 -> 15.7; S = 384
+// 1000 heads 77.5 -> 66.4, causal 62.0 -> 50.6; S = 512 128 heads 20.5 -> 19.8, causal 16.3 -> 15.1, causal 1000 heads
+// 82.4 -> 75.7; S = 1024 128 heads 54.8 -> 52.1, causal 12 heads 17.1 -> 14.5, causal 1000 heads 259 -> 256; S = 2000
+// causal 12 heads 29.6 -> 23.8.  Beyond the lines drawn here it loses: S = 1024 300 heads 111 -> 115, S = 2048 167 -> 180,
+// causal S = 2000 37 heads 35.6 -> 36.6, S = 2500 30 heads 42.4 -> 44.2, S = 2048 128 heads 101.6 -> 104.2; S = 449 to 512,
+// whose keys fill the pair's 128-key tiles, from 4000 tiles on, where the second reading of K and V tells (4096 heads 451 ->
+// 458; 1000 heads 113 -> 113; S = 448 wins at any size, 1000 heads 106 -> 94.5); causal S <= 160 (a second tile of a few
+// rows) 25.8 -> 26.5, and causal S <= 320 when pairs fill one wave but single tiles need second places on the SMs (66 heads
+// of S = 320 8.7 -> 9.2, 60 of S = 257 8.4 -> 8.9, 148 of S = 256 7.5 -> 8.2).  Inside them it loses up to 5 % at single
+// points whose pairs fill their last wave: 74 heads of S = 768 23.6 -> 24.8, 148 of S = 1000 61.9 -> 63.7, causal 41 of S =
+// 800 15.4 -> 16.1, 52 of S = 640 12.3 -> 12.8.
 bool single_tiles_pay(const FwdParams& p, int sm_count) {
   const long long heads = static_cast<long long>(p.B) * p.H;
   const long long tiles = heads * ((p.S + kRowsDb - 1) / kRowsDb), pairs = heads * ((p.S + 2 * kRowsDb - 1) / (2 * kRowsDb));
@@ -789,7 +791,7 @@ bool single_tiles_pay(const FwdParams& p, int sm_count) {
   if (!p.causal) return p.S <= 448 || (p.S <= 1024 && tiles <= (p.S <= 512 ? 27ll : 13ll) * sm_count);
   if (p.S <= 160 && tiles > sm_count) return false;
   if (p.S <= 320 && pairs <= sm_count && tiles > sm_count) return false;
-  return p.S <= 1024 || tiles <= 5ll * sm_count;
+  return p.S <= 1024 || tiles <= (p.S <= 1536 ? 5ll : 3ll) * sm_count;
 }
 
 cudaError_t launch_fwd_tcgen05_db_single(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {

@@ -4,6 +4,7 @@ Every case calls through the C ABI (ctypes -> rsfa_fwd).  Tolerance is the refer
 atol = rtol = 1e-2 (flash_attention_forward.py:736-738), plus a separate finiteness check
 because the reference's equal_nan=True would let NaN == NaN pass.
 """
+import contextlib
 import ctypes
 import math
 
@@ -25,6 +26,17 @@ def fa(cuda_device):
     mod.set_option("force_path", -1)
     yield mod
     mod.set_option("force_path", -1)
+
+
+@contextlib.contextmanager
+def kernel(fa, variant):
+    """The "tcgen05_variant" option: -1 by size, 0 the 128-key and 1 the 64-key kernel on pairs of Q tiles, 2 the
+    separate-P kernel (D <= 64).  By size, small launches run on other forms, whatever tile is requested."""
+    fa.set_option("tcgen05_variant", variant)
+    try:
+        yield
+    finally:
+        fa.set_option("tcgen05_variant", -1)
 
 
 def check(fa, q, k, v, causal, scale, bm, bn, dev, lse=True, tol=ATOL):
@@ -79,14 +91,19 @@ def test_reference_test_shapes(fa, cuda_device, Z, H, N, D, causal, BM, BN):
     assert m["max_abs"] < 4e-3  # the reference records <= 9.8e-4 on its shapes
 
 
-def test_bf16(fa, cuda_device):
-    # the reference's one bf16 case is (128, 8, 1024, 64), non-causal, tile (128, 128) (:698); 16 of its heads here
-    q, k, v = make_inputs(2, 8, 1024, 64, seed=20, std=0.5, dtype=torch.bfloat16)
-    check(fa, q, k, v, False, 0.5, 128, 128, cuda_device, tol=2e-2)
-    q, k, v = make_inputs(1, 2, 512, 128, seed=21, std=0.5, dtype=torch.bfloat16)
-    check(fa, q, k, v, True, 0.5, 128, 128, cuda_device, tol=2e-2)
-    q, k, v = make_inputs(1, 2, 100, 32, seed=22, std=0.5, dtype=torch.bfloat16)
-    check(fa, q, k, v, True, 0.5, 64, 64, cuda_device, tol=2e-2)
+@pytest.mark.parametrize("variant", [-1, 0, 1, 2])
+def test_bf16(fa, cuda_device, variant):
+    with kernel(fa, variant):
+        # the reference's one bf16 case is (128, 8, 1024, 64), non-causal, tile (128, 128) (:698); 16 of its heads here
+        q, k, v = make_inputs(2, 8, 1024, 64, seed=20, std=0.5, dtype=torch.bfloat16)
+        check(fa, q, k, v, False, 0.5, 128, 128, cuda_device, tol=2e-2)
+        q, k, v = make_inputs(1, 2, 512, 128, seed=21, std=0.5, dtype=torch.bfloat16)
+        check(fa, q, k, v, True, 0.5, 128, 128, cuda_device, tol=2e-2)
+        check(fa, q, k, v, False, 0.5, 128, 128, cuda_device, tol=2e-2)
+        q, k, v = make_inputs(1, 2, 1000, 128, seed=24, std=0.5, dtype=torch.bfloat16)
+        check(fa, q, k, v, True, 0.5, 128, 128, cuda_device, tol=2e-2)
+        q, k, v = make_inputs(1, 2, 100, 32, seed=22, std=0.5, dtype=torch.bfloat16)
+        check(fa, q, k, v, True, 0.5, 64, 64, cuda_device, tol=2e-2)
 
 
 @pytest.mark.parametrize("D", [16, 32, 64, 128, 256])
@@ -119,7 +136,9 @@ def test_small_head_dims_on_the_d64_kernels(fa, cuda_device, D, variant):
 @pytest.mark.parametrize("causal", [False, True])
 def test_ragged_sequence_lengths(fa, cuda_device, S, D, causal):
     q, k, v = make_inputs(1, 2, S, D, seed=S)
-    check(fa, q, k, v, causal, 0.25, 128, 128, cuda_device)
+    for variant in (-1,) if D == 256 else (-1, 0, 1) if D == 128 else (-1, 0, 1, 2):
+        with kernel(fa, variant):
+            check(fa, q, k, v, causal, 0.25, 128, 128, cuda_device)
 
 
 @pytest.mark.parametrize("path", [0, 1])
@@ -152,10 +171,9 @@ def test_both_tcgen05_variants(fa, cuda_device, variant, causal):
 
 @pytest.mark.parametrize("causal", [False, True])
 def test_short_sequences_on_both_kernel_families(fa, cuda_device, causal):
-    # Sequences of at most 128 keys run on the tcgen05 kernel, whatever the batch (one work item is a
-    # single, partly empty pair of Q tiles; HBM-bound for large batches), except D = 16 and S <= 64 at
-    # D <= 64, which stay on the short-sequence kernel.  The launch counter shows one launch either
-    # way (a single key tile does not use the D = 64 two-launch scheme).
+    # Sequences of at most 128 keys are one key tile: the kernel for that (S <= 128 at D <= 64, S <= 64 at D = 128) or
+    # a tcgen05 kernel with one key tile per Q tile, one launch either way.  select_path and work_items name the
+    # family, and count its items, by size alone.
     for B, H, S, D, scale in [(40, 8, 128, 128, 0.3), (33, 8, 96, 64, 0.25), (32, 8, 128, 256, 0.0625),
                               (64, 4, 77, 128, 0.3), (64, 4, 64, 64, 0.25), (2, 4, 128, 128, 0.3),
                               (64, 4, 128, 32, 0.3), (33, 8, 100, 16, 0.5), (64, 4, 64, 32, 0.3), (1, 1, 128, 128, 0.3),
@@ -174,12 +192,15 @@ def test_separate_p_kernel_repeats_items_whose_sum_check_failed(fa, cuda_device)
     # item whose sum check failed is run again by the same CTA with the loop that can.  Near one-hot rows
     # with a growing maximum (sm_scale 3) fail in many items; flat rows in none.  Both must match the
     # oracle, and each call is one launch.
+    # (By size these lengths run with one Q tile per CTA, which repairs in place: the same data for that.)
     q, k, v = make_inputs(2, 3, 1024, 64, seed=31)
-    n0 = fa.launch_count()
-    check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)
-    check(fa, q, k, v, True, 3.0, 128, 128, cuda_device)
-    check(fa, q, k, v, False, 0.125, 128, 128, cuda_device)
-    assert fa.launch_count() - n0 == 3
+    for variant in (2, -1):
+        with kernel(fa, variant):
+            n0 = fa.launch_count()
+            check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)
+            check(fa, q, k, v, True, 3.0, 128, 128, cuda_device)
+            check(fa, q, k, v, False, 0.125, 128, 128, cuda_device)
+            assert fa.launch_count() - n0 == 3
 
 
 @pytest.mark.parametrize("shape", [(1, 1, 256, 64), (1, 1, 300, 64), (1, 2, 129, 32), (1, 1, 777, 64), (3, 1, 513, 16)])
@@ -200,12 +221,14 @@ def test_separate_p_kernel_gives_up_on_the_fast_loop_for_one_hot_rows(fa, cuda_d
     # 512 work items, more than three per CTA: a CTA that has had to repeat more than one item in four
     # runs the rest of its items with the repairing loop at once.  Every item must still come out
     # right, whichever loop produced it; bf16 and a ragged length go through the same paths.
-    q, k, v = make_inputs(4, 64, 512, 64, seed=37)
-    check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)
-    check(fa, q, k, v, True, 3.0, 128, 128, cuda_device)
-    q, k, v = make_inputs(2, 40, 1000, 64, seed=38, dtype=torch.bfloat16)
-    check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)
-    check(fa, q, k, v, True, 3.0, 128, 128, cuda_device)
+    for variant in (2, -1):
+        with kernel(fa, variant):
+            q, k, v = make_inputs(4, 64, 512, 64, seed=37)
+            check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)
+            check(fa, q, k, v, True, 3.0, 128, 128, cuda_device)
+            q, k, v = make_inputs(2, 40, 1000, 64, seed=38, dtype=torch.bfloat16)
+            check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)
+            check(fa, q, k, v, True, 3.0, 128, 128, cuda_device)
 
 
 def test_repairing_loop_follows_a_maximum_that_keeps_growing(fa, cuda_device):
@@ -221,46 +244,58 @@ def test_repairing_loop_follows_a_maximum_that_keeps_growing(fa, cuda_device):
         q = (torch.randn(1, 2, S, D, generator=g).sign()).to(torch.float16)
         v = torch.randn(1, 2, S, D, generator=g).to(torch.float16)
         for causal in (False, True):
-            check(fa, q, k, v, causal, 1.0, 128, 128, cuda_device)
+            for variant in (2, -1):
+                with kernel(fa, variant):
+                    check(fa, q, k, v, causal, 1.0, 128, 128, cuda_device)
 
 
 def test_result_does_not_depend_on_requested_tile(fa, cuda_device):
     """Requests that resolve to the same instantiated tile are bit-identical; different tiles agree
-    within the tolerance (the reference's results are tile-independent in the same sense)."""
-    for D in (64, 128):
-        q, k, v = [t.to(cuda_device) for t in make_inputs(1, 2, 512, D, seed=4)]
+    within the tolerance (the reference's results are tile-independent in the same sense).  At sizes at which the
+    request decides: long rows, more of them than the forms for small launches take."""
+    for D, heads, S in ((64, 64, 2304), (128, 160, 1536)):
+        g = torch.Generator(device=cuda_device).manual_seed(4)
+        q, k, v = [torch.randn(1, heads, S, D, generator=g, device=cuda_device).half() for _ in range(3)]
         outs = {}
         for bm, bn in [(16, 16), (64, 32), (128, 64), (128, 128), (128, 512), (256, 256)]:
-            tile = fa.select_path(512, D, True, 0.5, bm, bn)[1:]
-            o = fa.attention(q, k, v, True, 0.5, bm, bn)
+            tile = fa.select_path(S, D, True, 0.125, bm, bn)[1:]
+            o = fa.attention(q, k, v, True, 0.125, bm, bn)
             torch.cuda.synchronize()
             if tile in outs:
                 assert torch.equal(o, outs[tile])
             outs[tile] = o
-        assert set(outs) == {(128, 64), (128, 128)}      # both instantiated tiles were reached
+        assert set(outs) == {(128, 64), (128, 128)}      # both instantiated tiles were asked for
+        for tile, variant in (((128, 64), 1), ((128, 128), 2 if D == 64 else 0)):
+            with kernel(fa, variant):                    # ... and ran
+                assert torch.equal(fa.attention(q, k, v, True, 0.125, *tile), outs[tile]), (D, tile)
         a, b = outs[(128, 64)].float(), outs[(128, 128)].float()
-        assert torch.allclose(a, b, atol=ATOL, rtol=RTOL)
+        assert not torch.equal(a, b) and torch.allclose(a, b, atol=ATOL, rtol=RTOL)
 
 
 def test_wide_logits_online_softmax_stability(fa, cuda_device):
     # the cfg5 recipe: inputs x2 widen the logit range; also a huge-scale case that forces rescales
     q, k, v = make_inputs(1, 2, 2048, 64, seed=8, std=2.0)
-    check(fa, q, k, v, True, 0.125, 128, 128, cuda_device)
-    check(fa, q, k, v, False, 0.125, 128, 128, cuda_device)
+    for variant in (2, 1, -1):
+        with kernel(fa, variant):
+            check(fa, q, k, v, True, 0.125, 128, 128, cuda_device)
+            check(fa, q, k, v, False, 0.125, 128, 128, cuda_device)
     q, k, v = make_inputs(1, 1, 1024, 128, seed=8, std=1.0)
-    check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)   # near one-hot rows, max keeps growing
+    for variant in (0, 1, -1):
+        with kernel(fa, variant):
+            check(fa, q, k, v, False, 3.0, 128, 128, cuda_device)   # near one-hot rows, max keeps growing
     # keys sorted so every tile raises the running max: exercises the in-TMEM rescale each step
     kn = k.float().norm(dim=-1)
     order = kn.argsort(dim=-1)
     k2 = torch.gather(k, 2, order[..., None].expand_as(k))
     q2 = k2.flip(2).contiguous()
-    check(fa, q2, k2, v, False, 1.0, 128, 128, cuda_device)
+    for variant in (0, 1, -1):
+        with kernel(fa, variant):
+            check(fa, q2, k2, v, False, 1.0, 128, 128, cuda_device)
 
 
 @pytest.mark.parametrize("causal", [False, True])
-@pytest.mark.parametrize("tile", [(128, 128), (128, 64)])
-@pytest.mark.parametrize("D", [64, 128])
-def test_sudden_growth_of_the_row_maximum(fa, cuda_device, causal, tile, D):
+@pytest.mark.parametrize("D,variant", [(64, -1), (64, 0), (64, 1), (64, 2), (128, -1), (128, 0), (128, 1)])
+def test_sudden_growth_of_the_row_maximum(fa, cuda_device, causal, D, variant):
     # The kernels exponentiate a key tile against a reference fixed at the first tile and move
     # it only when a value might leave the 16-bit range of P.  Flat scores everywhere except a
     # few keys that beat everything before them by far more than that range: one in the second
@@ -273,12 +308,14 @@ def test_sudden_growth_of_the_row_maximum(fa, cuda_device, causal, tile, D):
     v = torch.randn(B, H, S, D, generator=g).half()
     for idx, c in ((128 + 70, 40.0), (256 + 10, 90.0), (512 + 100, 150.0)):
         k[:, :, idx, :] = (c * u).half()
-    m = check(fa, q, k, v, causal, 0.5, tile[0], tile[1], cuda_device)
+    with kernel(fa, variant):
+        m = check(fa, q, k, v, causal, 0.5, 128, 128, cuda_device)
     assert m["max_abs"] < 4e-3, m
     # moderate growth (a few log2 units per tile) must stay on the fast path and stay exact too
     k2 = (0.3 * torch.randn(B, H, S, D, generator=g)).half()
     k2 *= torch.linspace(0.5, 3.0, S)[None, None, :, None].half()
-    m = check(fa, q, k2, v, causal, 0.5, tile[0], tile[1], cuda_device)
+    with kernel(fa, variant):
+        m = check(fa, q, k2, v, causal, 0.5, 128, 128, cuda_device)
     assert m["max_abs"] < 4e-3, m
 
 
@@ -334,14 +371,17 @@ def test_cfg4_shape_long_sequence_d128(fa, cuda_device, causal):
     bm, bn = fa.get_tiling(16, 16, 4096, 128, causal)
     m = _check_config_shape(fa, cuda_device, "cfg4", 2, 4, causal, bm, bn)
     assert m["max_abs"] < 4e-3, m          # N(0,1) inputs: outputs of order 1
-    _check_config_shape(fa, cuda_device, "cfg4", 2, 4, causal, 128, 64)   # the 64-key kernel at 64 key tiles per row
+    for variant in (0, 1):                 # pairs of Q tiles: 128-key tiles, and 64 key tiles of 64 per row
+        with kernel(fa, variant):
+            _check_config_shape(fa, cuda_device, "cfg4", 2, 4, causal, bm, bn)
 
 
 @pytest.mark.parametrize("variant", [-1, 0, 1, 2])
 @pytest.mark.parametrize("causal", [False, True])
 def test_cfg5_shape_very_long_small_head_wide_logits(fa, cuda_device, causal, variant):
-    # 64 key tiles of 128 per row; variant -1 / 2 = separate-P kernel, 0 = 128-key kernel, 1 = 64-key
-    # kernel: one launch each.  Inputs x 2.0 widen the logits (std 5.8 log2 units).
+    # 64 key tiles of 128 per row; variant 2 = separate-P kernel, 0 = 128-key kernel, 1 = 64-key kernel, -1 = by size:
+    # separate-P, with the mask (four heads) one Q tile per CTA.  One launch each.  Inputs x 2.0 widen the logits (std
+    # 5.8 log2 units).
     fa.set_option("tcgen05_variant", variant)
     try:
         n0 = fa.launch_count()
@@ -352,8 +392,8 @@ def test_cfg5_shape_very_long_small_head_wide_logits(fa, cuda_device, causal, va
 
 
 def test_more_heads_than_a_grid_dimension_on_the_short_sequence_kernel(fa, cuda_device):
-    # 8192 x 16 = 131072 heads of S=64, D=64: the short-sequence kernel keeps its heads on grid.x
-    # (gridDim.y would stop at 65535).  q = k = 0 gives uniform weights, v = 1 gives O = 1 everywhere.
+    # 8192 x 16 = 131072 heads of S=64, D=64: the kernel for a single key tile walks over them, and the general kernel
+    # keeps them on grid.x (gridDim.y would stop at 65535).  q = k = 0 gives uniform weights, v = 1 gives O = 1.
     from ascend_rsfa import _capi
 
     B, H, S, D = 8192, 16, 64, 64
@@ -363,15 +403,22 @@ def test_more_heads_than_a_grid_dimension_on_the_short_sequence_kernel(fa, cuda_
     z = torch.zeros(B, H, S, D, dtype=torch.float16, device=cuda_device)
     v = torch.ones_like(z)
     v[-1, -1] = 3.0                      # the very last head is told apart
-    for causal in (False, True):
-        o = fa.attention(z, z, v, causal, 0.5, 64, 64)
-        torch.cuda.synchronize()
-        assert bool((o[:-1] == 1).all()) and bool((o[-1, :-1] == 1).all()) and bool((o[-1, -1] == 3).all())
+    for path in (-1, 0):
+        fa.set_option("force_path", path)
+        try:
+            for causal in (False, True):
+                o = fa.attention(z, z, v, causal, 0.5, 64, 64)
+                torch.cuda.synchronize()
+                assert bool((o[:-1] == 1).all()) and bool((o[-1, :-1] == 1).all()) and bool((o[-1, -1] == 3).all())
+        finally:
+            fa.set_option("force_path", -1)
     del z, v, o
     torch.cuda.empty_cache()
 
 
-def test_bounded_wait_runs_out_and_is_reported(fa, cuda_device):
+@pytest.mark.parametrize("heads,S,variant,load", [(1, 256, -1, 1), (1, 256, 0, 1), (3, 512, 0, 2), (160, 512, 0, 3), (3, 640, 0, 5),
+                                                  (3, 512, -1, 2), (300, 100, -1, 0), (300, 100, -1, 1)])
+def test_bounded_wait_runs_out_and_is_reported(fa, cuda_device, heads, S, variant, load):
     """The wait-expired path on a healthy GPU: the producer leaves out one K/V tile load together
     with the barrier arrival that would announce it (the "test_drop_load" option), so nothing is in
     flight and no address is touched; the MMA warp's wait for that tile runs out after
@@ -380,29 +427,33 @@ def test_bounded_wait_runs_out_and_is_reported(fa, cuda_device):
     from ascend_rsfa import _capi
 
     lib = _capi.load()
-    q, k, v = [t.to(cuda_device) for t in make_inputs(1, 1, 256, 128, seed=3)]
-    ref = attention_fp32(q.cpu(), k.cpu(), v.cpu(), False, 0.5)
-    fa.device_status()                                   # clean before the experiment
-    fa.set_option("wait_limit_ms", 1)
-    fa.set_option("test_drop_load", 1)                   # load 0 = K_0, load 1 = V_0
-    try:
-        fa.attention(q, k, v, False, 0.5, 128, 128)      # returns normally: the launch is asynchronous
-        torch.cuda.synchronize()
-    finally:
-        fa.set_option("test_drop_load", -1)
-        fa.set_option("wait_limit_ms", 2000)
-    raw = ctypes.c_int(0)
-    rc = lib.rsfa_device_status(0, ctypes.byref(raw))
-    assert rc == _capi.RSFA_ERR_DEVICE_STATUS
-    assert (raw.value >> 16) == 1 and 1 <= (raw.value & 0xffff) <= 10, hex(raw.value)
-    assert lib.rsfa_device_status(0, ctypes.byref(raw)) == _capi.RSFA_OK and raw.value == 0   # reading cleared it
-    # the context is intact and the next ordinary calls are correct (the work queue was left clean)
-    for _ in range(2):
-        o = fa.attention(q, k, v, False, 0.5, 128, 128)
-        torch.cuda.synchronize()
-        m = error_metrics(o, ref)
+    # by size these are split keys and two heads per item; variant 0 is the pair form, whose loads are K_0 V_0 K_1 V_1 ...,
+    # counted with the hand-overs of P: K_0 alone, V_0 with the first half, K_1 with the second, and steps further on
+    q, k, v = [t.to(cuda_device) for t in make_inputs(1, heads, S, 128, seed=3)]
+    with kernel(fa, variant):
+        ref = fa.attention(q, k, v, False, 0.5, 128, 128)
+        fa.device_status()                               # clean before the experiment
+        m = error_metrics(ref[:, :3], attention_fp32(q[:, :3].cpu(), k[:, :3].cpu(), v[:, :3].cpu(), False, 0.5))
         assert m["finite"] and m["allclose"], m
-    fa.device_status()
+        fa.set_option("wait_limit_ms", 1)
+        fa.set_option("test_drop_load", load)
+        try:
+            fa.attention(q, k, v, False, 0.5, 128, 128)  # returns normally: the launch is asynchronous
+            torch.cuda.synchronize()
+        finally:
+            fa.set_option("test_drop_load", -1)
+            fa.set_option("wait_limit_ms", 2000)
+        raw = ctypes.c_int(0)
+        rc = lib.rsfa_device_status(0, ctypes.byref(raw))
+        assert rc == _capi.RSFA_ERR_DEVICE_STATUS
+        assert (raw.value >> 16) == 1 and 1 <= (raw.value & 0xffff) <= 10, hex(raw.value)
+        assert lib.rsfa_device_status(0, ctypes.byref(raw)) == _capi.RSFA_OK and raw.value == 0   # reading cleared it
+        # the context is intact and the next ordinary calls are correct (the work queue was left clean)
+        for _ in range(2):
+            o = fa.attention(q, k, v, False, 0.5, 128, 128)
+            torch.cuda.synchronize()
+            assert torch.equal(o, ref)
+        fa.device_status()
 
 
 def test_check_status_option_makes_the_next_call_fail(fa, cuda_device):
@@ -444,16 +495,18 @@ def test_d64_calls_on_several_streams_keep_their_repeats_apart(fa, cuda_device):
     qd, kd, vd = [t.to(cuda_device) for t in (q, k, v)]
     streams = [torch.cuda.Stream(device=cuda_device) for _ in range(3)]
     torch.cuda.synchronize()
-    outs = []
-    for i in range(24):
-        causal = bool(i & 1)
-        with torch.cuda.stream(streams[i % 3]):
-            outs.append((causal, fa.attention(qd, kd, vd, causal, 3.0, 128, 128)))
-    torch.cuda.synchronize()
-    fa.device_status()
-    for causal, o in outs:
-        m = error_metrics(o, ref[causal])
-        assert m["finite"] and m["allclose"], m
+    for variant in (2, -1):      # -1: one Q tile per CTA, which repairs in place
+        outs = []
+        with kernel(fa, variant):
+            for i in range(24):
+                causal = bool(i & 1)
+                with torch.cuda.stream(streams[i % 3]):
+                    outs.append((causal, fa.attention(qd, kd, vd, causal, 3.0, 128, 128)))
+            torch.cuda.synchronize()
+        fa.device_status()
+        for causal, o in outs:
+            m = error_metrics(o, ref[causal])
+            assert m["finite"] and m["allclose"], m
 
 
 def test_back_to_back_launches_of_mixed_shapes_on_two_streams(fa, cuda_device):

@@ -46,6 +46,33 @@ def test_lengths_at_the_edges_of_strips_and_steps(fa, cuda_device, D, heads, dty
             assert torch.allclose(lse.cpu(), lse_ref, atol=1e-4, rtol=1e-4), (S, causal)
 
 
+@pytest.mark.parametrize("D,S,heads", [(16, 16, 40000), (16, 32, 40000), (16, 100, 12000), (16, 128, 12000), (32, 16, 40000),
+                                       (32, 30, 20000), (32, 64, 20000), (32, 128, 4000), (64, 16, 20000), (64, 30, 20000),
+                                       (64, 64, 6000), (128, 16, 8000)])
+def test_ring_slots_used_again_and_again(fa, cuda_device, D, S, heads):
+    # at least twice as many rounds as a ring has slots, one to eight warps per team: the last reader's refill, the phase
+    # of the slot and the count of its readers; every head against the general kernel, three rounds' against the oracle
+    strips = -(-S // 16)
+    tile = -(-S // 32) * 32 * D * 2
+    teams = min(8 // strips, 98304 // (3 * tile))
+    stages = min(8, 98304 // (teams * 3 * tile))
+    assert -(-heads // (2 * torch.cuda.get_device_properties(0).multi_processor_count * teams)) >= 2 * stages + 1
+    g = torch.Generator(device=cuda_device).manual_seed(D + S)
+    q, k, v = [torch.randn(heads // 4, 4, S, D, generator=g, device=cuda_device).half() for _ in range(3)]
+    scale = 1.0 / math.sqrt(D)
+    for causal in (False, True):
+        o = fa.attention(q, k, v, causal, scale, 64, 64)
+        fa.set_option("force_path", 0)
+        try:
+            general = fa.attention(q, k, v, causal, scale, 64, 64)
+        finally:
+            fa.set_option("force_path", -1)
+        assert float((o.float() - general.float()).abs().max()) <= 2 * bound(v, torch.float16), causal
+        for b in (0, heads // 8, heads // 4 - 1):
+            ref = attention_fp32(*(t[b:b + 1].cpu() for t in (q, k, v)), causal, scale)
+            assert float((o[b:b + 1].cpu().float() - ref).abs().max()) <= bound(v[b:b + 1], torch.float16), (b, causal)
+
+
 @pytest.mark.parametrize("S,D", [(64, 64), (50, 128), (100, 32), (128, 16), (23, 64)])
 def test_storage_orders_agree_with_the_general_kernel(fa, cuda_device, S, D):
     B, H = 5, 6
