@@ -31,8 +31,9 @@ struct FwdParams {
   unsigned long long wait_limit_ns;
   int pdl;             // 1: launch with programmatic stream serialisation (the "pdl" option)
   // Test hook (the "test_drop_load" option, -1 = off): the producer of the 128-key tcgen05 kernel
-  // leaves out its n-th K/V tile load together with the barrier arrival that announces it, and the kernel
-  // for a single key tile the loads of head n.  Nothing is in flight for that tile and no address is touched; the consumer's bounded wait simply runs
+  // leaves out its n-th K/V tile load together with the barrier arrival that announces it, and the
+  // kernel for a single key tile those of the heads from n on among the loads it starts with.  Nothing
+  // is in flight for that tile and no address is touched; the consumer's bounded wait simply runs
   // out, which is how the tests reach the wait-expired path on a healthy GPU.
   int test_drop_load;
 #ifdef RSFA_TRACE

@@ -23,11 +23,13 @@
 // Measured on 4096 heads (us per launch from a graph of launches, inputs rotated; before = the kernel that had
 // the size: fwd_generic at S <= 64, D <= 64 and D = 16, the tcgen05 kernels otherwise; floor = bytes at the
 // measured copy rate, 6.55 TB/s):
-//   S = 64 D = 64     72.3 -> 23.0 (floor 20.5)     S = 64 D = 128        95.5 -> 48.5 (floor 41.0)
-//   S = 100 D = 32    84.0 -> 40.1 (floor 16.0)     the same, causal      84.0 -> 31.6
-//   S = 128 D = 64    72.5 -> 64.9 (floor 41.0)     the same, causal      84.8 -> 51
-//   S = 128 D = 16    57.3 -> 29.5 (floor 10.2)     S = 30 D = 64 (x 2)  109.9 -> 22.6 (floor 19.2)
-// and at 2 to 64 heads, where latency is all there is: S = 128 D = 64 5.7 -> 4.1, S = 64 D = 128 6.8 -> 3.5.
+//   S = 64 D = 64     72.3 -> 23.3 (floor 20.5)     S = 64 D = 128        95.5 -> 49.0 (floor 41.0)
+//   S = 100 D = 32    84.0 -> 40.2 (floor 16.0)     the same, causal      84.0 -> 32.5
+//   S = 128 D = 64    72.5 -> 67.0 (floor 41.0)     the same, causal      84.8 -> 51.5
+//   S = 128 D = 16    57.3 -> 31.6 (floor 10.2)     S = 30 D = 64 (x 2)  109.9 -> 22.6 (floor 19.2)
+// and at 2 heads, where latency is all there is: S = 128 D = 64 5.2 -> 4.3, S = 64 D = 128 6.2 -> 3.2.  At S = 128 D = 64
+// without the mask a launch whose heads just miss whole waves of two per SM is up to 3 % slower than on the tcgen05
+// kernel (300 heads 10.9 -> 11.3, 600 15.4 -> 15.9), a full wave 4 to 8 % faster.
 #include "../../include/rsfa.h"
 #include "tcgen05_common.cuh"
 
@@ -45,6 +47,7 @@ struct ShortMaps {
 
 struct ShortPlan {
   int heads;       // B * H
+  int first_loads; // heads whose loads a ring may start with: all, but for the test of a wait that runs out
   int strips;      // warps per team = ceil(S / 16)
   int teams;       // teams per CTA
   int stages;      // ring slots per team
@@ -149,7 +152,6 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
   };
   // one lane: Q, K and V of head `bh` into a slot of this team
   auto load_head = [&](int bh, int slot) {
-    if (bh == p.test_drop_load) return;   // test hook: this head is never announced
     const uint32_t bar = smem_u32(&full_bar[team * plan.stages + slot]);
     const uint32_t dst = ring + slot * slot_bytes;
     const int b = batch_of(bh), h = bh - b * p.H;
@@ -163,7 +165,7 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
   };
   if (strip == 0 && lane == 0) {
     for (int s = 0; s < plan.stages; ++s)
-      if (first + s * stride < plan.heads) load_head(first + s * stride, s);
+      if (first + s * stride < plan.first_loads) load_head(first + s * stride, s);
   }
   __syncwarp();
 
@@ -254,9 +256,9 @@ fwd_short_kernel(const __grid_constant__ ShortMaps maps, const FwdParams p, cons
     // The maximum comes off before the scale goes on: exact where it counts, whatever the scores' size.  With s * scale -
     // (m * scale) in one operation every P of the row is off by a factor 2^e, e the rounding error of m * scale; the
     // division takes it out again, but from products of 2^28 (fp16) and 2^31 (fp32) on P does not hold it: rows whose
-    // keys a program hides with the type's lowest value came out as NaN.  The second operation costs 0 to 2 % (4096 heads,
-    // us: S = 100 D = 32 40.1 -> 40.5, S = 64 D = 64 23.1 -> 23.1, S = 128 D = 64 66.1 -> 67.5, S = 64 D = 128 49.5 -> 49.7);
-    // a branch for large rows only costs the same or more (the best form of it 7 % on S = 64 D = 128 causal).
+    // keys a program hides with the type's lowest value came out as NaN.  The second operation costs 0 to 3 %, 5 % at most
+    // (4096 heads, us: S = 64 D = 64 23.3 -> 23.4, S = 100 D = 32 causal 31.8 -> 32.5, S = 128 D = 64 66.2 -> 67.7, S = 128
+    // D = 16 30.7 -> 31.6, S = 112 D = 16 30.0 -> 31.5); a branch for large rows only costs as much or more (S = 64 D = 128 7 %).
     // A row of nothing but -inf has the sum 0.
     const float ref_lo = m_lo == -INFINITY ? 0.f : m_lo, ref_hi = m_hi == -INFINITY ? 0.f : m_hi;
 
@@ -385,6 +387,7 @@ template <int D, int kKeys, bool kBf16, bool kAll>
 cudaError_t launch_short_one(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
   ShortPlan plan;
   plan.heads = p.B * p.H;
+  plan.first_loads = (p.test_drop_load >= 0 && p.test_drop_load < plan.heads) ? p.test_drop_load : plan.heads;
   plan.strips = (p.S + 15) / 16;
   const int rows = (p.S + 31) / 32 * 32;   // keys are taken 32 at a time; rows past S read as zeros
   plan.tile_bytes = rows * D * 2;
@@ -425,7 +428,7 @@ cudaError_t launch_short_one(const FwdParams& p, int sm_count, cudaStream_t stre
 // as many as the length needs, in steps of 32 keys (4096 heads, us: S = 100 D = 32 42.1 -> 40.1, S = 112 D = 16 33.4 ->
 // 29.5, S = 90 D = 64 46.1 -> 42.3, S = 20 D = 32, 8192 heads, 12.6 -> 11.9).  Not at D = 64 with 128 keys, where the
 // straight line spills (64.9 -> 66.8), and not with fewer than 64 keys' registers for causal rows of D >= 64 (S = 30
-// 21.9 -> 22.4).
+// 21.9 -> 22.4).  These figures are from before the maximum came off the scores in an operation of its own.
 template <int D, int kKeys>
 cudaError_t launch_short_keys(const FwdParams& p, int sm_count, cudaStream_t stream, long long* launches) {
   if constexpr (D < 64 || kKeys < 128) {

@@ -187,8 +187,8 @@ RSFA_API long long rsfa_launch_count(void);
  * the kernel in front of it on the stream; they wait for that kernel before touching global memory),
  * "check_status" (0 / 1, see rsfa_device_status), "test_drop_load" (-1 = off; n >= 0: every CTA of the
  * 128-key tcgen05 kernel leaves out its n-th K/V tile load and the barrier arrival that announces it, and
- * the kernel for a single key tile the loads of head n (of B * H), so that a bounded wait runs out - for
- * tests of the wait-expired path; the output of such a call is incomplete).
+ * the kernel for a single key tile, of the loads that it starts with, those of the heads from n on (of B * H),
+ * so that a bounded wait runs out - for tests of the wait-expired path; the output of such a call is incomplete).
  * rsfa_get_option also answers "workspace_devices": the number of devices on which rsfa_fwd has
  * created its workspace (0 in a process that has only used rsfa_fwd_noalloc).
  * Unknown names -> RSFA_ERR_INVALID_ARGUMENT.

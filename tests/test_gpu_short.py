@@ -142,10 +142,10 @@ def test_scores_of_any_size(fa, cuda_device, D, hide):
                 assert float((o.cpu().float() - ref).abs().max()) <= bound(v, torch.bfloat16), (S, causal)
 
 
-@pytest.mark.parametrize("B,H,S,D,head", [(5, 6, 100, 64, 7), (400, 4, 64, 128, 1599), (3000, 4, 16, 16, 11000)])
+@pytest.mark.parametrize("B,H,S,D,head", [(5, 6, 100, 64, 7), (400, 4, 64, 128, 500), (3000, 4, 16, 16, 9000)])
 def test_a_wait_that_runs_out_is_reported(fa, cuda_device, B, H, S, D, head):
-    """The loads of one head and the arrival that announces them are left out ("test_drop_load"): nothing is in flight and
-    no address is touched, the wait of the team that owns the head runs out and the kernel returns by itself."""
+    """Of the first loads, those of the heads from one on and the arrivals that announce them are left out ("test_drop_load"): nothing is in
+    flight and no address is touched, the waits of the teams that own them run out and the kernel returns by itself."""
     from ascend_rsfa import _capi
 
     lib = _capi.load()
@@ -153,7 +153,7 @@ def test_a_wait_that_runs_out_is_reported(fa, cuda_device, B, H, S, D, head):
     whole = fa.attention(q, k, v, False, 0.2, 64, 64)
     fa.device_status()
     fa.set_option("wait_limit_ms", 1)
-    fa.set_option("test_drop_load", head)     # the first head of a team, and ones that go to slots used before
+    fa.set_option("test_drop_load", head)     # from the first slots of the rings, and from their last ones
     try:
         fa.attention(q, k, v, False, 0.2, 64, 64)
         torch.cuda.synchronize()
