@@ -78,7 +78,7 @@ struct Cfg {
   static constexpr int kQTileBytes = kTileM * D * 2;
   static constexpr int kQBufs = (kMode == kSplitKeys) ? 1 : kNT;   // its two tiles have the same rows
   static constexpr int kKvTileBytes = kTileN * D * 2;
-  static constexpr int kStages = 4;
+  static constexpr int kStages = 4;   // two steps ahead: as far as the turns of the shared barriers reach (bar_p_full)
   static constexpr int kQBoxBytes = kTileM * 128;             // 128 rows x 128 B
   static constexpr int kKvBoxBytes = kTileN * 128;
   static constexpr int kStageBytes = kTileM * 128;            // epilogue staging: 128 rows x 64 columns
@@ -119,8 +119,9 @@ fwd_tcgen05_kernel(const __grid_constant__ TmaMaps maps, const FwdParams p, cons
   // same barriers and one wait says both; with K/V tiles shared by the Q tiles (kPair) on those of tile 0.  The
   // loads run up to two steps ahead of the softmax: such barriers are two pairs used in turn (`step` = the key
   // tiles of that Q tile so far).  Two waits per step less (four instead of six for the warp that paces the CTA):
-  // (16, 16, 4096, 128) causal 911 -> 894 us, (128, 8, 2048, 128) 1925 -> 1877, S = 1024 causal 86.6 -> 84.7, 8 heads
-  // of S = 2048 (kSplitKeys) 22.4 -> 21.6.
+  // 2 % in bursts at full clock ((16, 16, 4096, 128) causal 911 -> 894 us, S = 1024 causal 86.6 -> 84.7, 8 heads of
+  // S = 2048 (kSplitKeys) 22.4 -> 21.6); under the power cap, where the large shapes run back to back, 1 % at most
+  // ((128, 8, 2048, 128) 1967 -> 1955 us and the causal shape 1027 -> 1019 with all that changed around it).
   auto joint = [](int t) { return kMode != kPair || t == 0; };
   auto bar_p_full = [&](int t, int half, uint32_t step) {
     return (joint(t) && (step & 1) != 0) ? sBar + 8u * (C::kNumBarriers - 2 * kNT + 2 * t + half)

@@ -56,8 +56,9 @@ struct DbCfg {
   // One Q tile: the bytes of the ring entry that a step needs, (V_j, K_{j+2}), are counted on the barrier on which
   // the softmax hands over P_j, so the MMA warp waits once per step.  The loads run up to kStages entries ahead of
   // the softmax: kTurns such barriers are used in turn (kTurns >= kStages: a barrier's turn comes again when the
-  // ring slot of the step that had it is given back).  D = 256: S = 1024 causal 321 -> 308 us, S = 2048 causal 542 ->
-  // 512; D = 64 1 %.  (One MMA warp for a pair of tiles, which could have the same, is 5 % slower: 24 MMAs and
+  // ring slot of the step that had it is given back).  In bursts, D = 256: S = 1024 causal 321 -> 308 us, S = 2048 causal
+  // 542 -> 512; D = 64 1 %.  In a stream of calls S = 1024 causal went from 382 to 366 us with this, the WorkItem ring and
+  // the early claim together.  (One MMA warp for a pair of tiles, which could have the same, is 5 % slower: 24 MMAs and
   // their commits per step are more than one warp can issue.)
   static constexpr bool kJoint = (NT == 1);
   static constexpr int kTurns = kJoint ? 4 : 0;

@@ -82,11 +82,13 @@ int ensure_device(int device, DeviceState** out) {
 
 bool valid_head_dim(int D) { return D == 16 || D == 32 || D == 64 || D == 128 || D == 256; }
 
-// Kernel family by shape (a single key tile then runs on fwd_short.cu in either family's place, see
-// short_fits; the times below are the families' own).  The tcgen05 kernels take everything they are instantiated for (sm_scale > 0)
-// except the smallest tiles: head dimension 16, and sequences of at most 64 keys at D <= 64, stay on
-// the short-sequence kernel, the counterpart of the reference's single-tile kernels for N_CTX <= 128
-// (:564).  Measured per call, host clock around call + synchronise / 4096 heads back to back:
+// Kernel family by shape.  With sm_scale > 0 the line between the families only names: it is what
+// rsfa_select_path, rsfa_get_tiling and rsfa_work_items answer by, and where calls go that set
+// "tcgen05_variant".  A sequence of one key tile runs on fwd_short.cu whichever family it belongs to
+// (short_fits, asked in rsfa_fwd); what is left of the general family are the shapes with sm_scale <= 0.
+// The line lies where the two families' own times crossed before that kernel (head dimension 16 at S <= 128,
+// and at most 64 keys at D <= 64, were faster on the general one, the counterpart of the reference's
+// single-tile kernels for N_CTX <= 128, :564).  Per call, host clock around call + synchronise / 4096 heads back to back:
 //   S = 128 D = 128: 34 against 44 us at 128 heads, 93 against 346 us at 4096 (HBM rate against not);
 //   S = 128 D = 64: 33 against 41 us; D = 256: 34 against 52 us; S = 128 D = 32: 66 against 107 us at 4096;
 //   S = 64 D = 64: 32 against 34 us at 128 heads but 78 against 74 us at 4096; S = 64 D = 32: 77 against 38 us;

@@ -1,6 +1,7 @@
-"""The two forms of the D = 128 kernel in which each Q tile of a CTA has K/V tiles of its own - two heads per
-work item (S <= 128), and the keys of one block of rows dealt out to both tiles - on a B200 against the fp32
-oracle, at the sizes where their bookkeeping can go wrong."""
+"""The forms of the tcgen05 kernels for launches that pairs of Q tiles do not suit, on a B200 at the sizes where their
+bookkeeping can go wrong: the two of the D = 128 kernel in which each Q tile of a CTA has K/V tiles of its own - two
+heads per work item (S <= 128), and the keys of one block of rows dealt out to both tiles - and one Q tile per CTA at
+D <= 64.  Against the fp32 oracle, the pair kernels and the general kernel."""
 import math
 
 import pytest
