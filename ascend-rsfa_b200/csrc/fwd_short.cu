@@ -28,8 +28,8 @@
 //   S = 128 D = 64    72.5 -> 67.0 (floor 41.0)     the same, causal      84.8 -> 51.5
 //   S = 128 D = 16    57.3 -> 31.6 (floor 10.2)     S = 30 D = 64 (x 2)  109.9 -> 22.6 (floor 19.2)
 // and at 2 heads, where latency is all there is: S = 128 D = 64 5.2 -> 4.3, S = 64 D = 128 6.2 -> 3.2.  At S = 128 D = 64
-// without the mask a launch whose heads just miss whole waves of two per SM is up to 3 % slower than on the tcgen05
-// kernel (300 heads 10.9 -> 11.3, 600 15.4 -> 15.9), a full wave 4 to 8 % faster.
+// without the mask a launch whose heads leave the last wave of two per SM thin is up to 4 % slower than on the tcgen05
+// kernel (300 heads 10.9 -> 11.3, 600 15.4 -> 15.9, 1000 21.7 -> 22.4), one of full waves 4 to 8 % faster.
 #include "../../include/rsfa.h"
 #include "tcgen05_common.cuh"
 
